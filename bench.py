@@ -371,6 +371,7 @@ def run_b200_arm(args, wm, world, rank, local):
             "bound": "hbm",
             "kernel": ("step kernels: tile_step_kernel (+ warp_step_kernel on the CTAs that meet a CPML slab) "
                        "+ ade_pass_kernel (one step)") if info1["variant"] == 10 else
+                      "step kernels: quad_step_kernel + ade_pass_kernel (one step)" if info1["variant"] == 11 else
                       "step kernels: warp_step_kernel + ade_pass_kernel (one step)",
             "achieved": achieved,
             "peak": peaks["hbm_gbs"],

@@ -249,21 +249,24 @@ int fdtd_engine_autotune(fdtd_engine* h, int* tile_rows, int* chunk_planes);
  * warps and a halo warp per CTA sharing y-neighbour rows through shared
  * memory; with CPML in the scene the CTAs that meet a slab run in the warp
  * kernel of variant 2 after it; poles run in the ADE pass, and variant 2 runs
- * in its place where that pass cannot take them).  Default: 10 for FP32
- * engines without CPML, periodic or Bloch faces, 2 otherwise; reduced storage
- * runs 2 only.
+ * in its place where that pass cannot take them); 11: the quad-tile kernel (four
+ * z cells per thread, whole z rows copied in bulk, CPML and wrapped faces
+ * included; up to 512 z nodes and 24 injection terms, no PMC faces; poles as with
+ * 10).  Default: 11 for FP32 engines it takes; else 10 without CPML, periodic, Bloch
+ * or PMC faces, 2 otherwise; reduced storage runs 2 only.
  * chunk_planes is the number of x planes each warp marches through (0 picks
- * the variant's default).  tile_rows is accepted for compatibility and
- * ignored. */
+ * the variant's default).  tile_rows is the number of rows of a CTA of variant 11
+ * (0 picks its default; FDTD_ERR_INVALID_ARG when a CTA cannot hold them); the
+ * other variants ignore it.  Autotuning an engine that runs 11 picks its tile. */
 int fdtd_engine_set_launch(fdtd_engine* h, int variant, int tile_rows, int chunk_planes);
 int fdtd_engine_get_launch(fdtd_engine* h, int* variant, int* tile_rows, int* chunk_planes);
 /* Where the Debye / Drude / Lorentz poles advance: on (1, the default) in a
  * separate streaming pass after the step kernel, over the cells the pole boxes
  * cover, in the reference's order (E update, TFSF and source terms, then the
  * dispersive correction: witwin/maxwell/fdtd/runtime/stepping.py:2290-2316);
- * off (0) inside the fused step kernel.  The pass is used with FP32 storage,
- * launch variants 1-3 and no periodic / Bloch face; elsewhere the poles stay
- * in the step kernel.  The two orders agree to FP32 rounding. */
+ * off (0) inside the fused step kernel.  The pass is used with FP32 storage and
+ * launch variants 1-3 and 10 without periodic / Bloch faces, or 11; elsewhere the
+ * poles stay in the step kernel.  The two orders agree to FP32 rounding. */
 int fdtd_engine_set_ade_pass(fdtd_engine* h, int on);
 /* L2 prefetch distance of the scalar step kernels (variants 1-3; default 2):
  * warps whose footprint has no CPML and no coefficient-array cell prefetch
@@ -273,8 +276,8 @@ int fdtd_engine_set_prefetch(fdtd_engine* h, int planes);
 /* Failure detection: polling rounds (default 1 << 20) a bounded pipeline wait
  * inside a step kernel makes before it gives up, records FDTD_ERR_TIMEOUT in
  * the device status word and returns; the next step_range then returns
- * FDTD_ERR_TIMEOUT.  The TMA variant (4) waits on its mbarrier ring this way;
- * its producer still waits for every copy it issued before the block exits
+ * FDTD_ERR_TIMEOUT.  Variants 4, 10 and 11 wait on their mbarrier rings this way;
+ * their producer still waits for every copy it issued before the block exits
  * (that drain has its own fixed bound).  0 makes every pipeline wait run out
  * at once, which is how the timeout path is tested.  No counterpart in the
  * reference (its kernels have no device-side waits). */
@@ -319,7 +322,7 @@ int fdtd_batch_info(fdtd_batch* b, int* n_engines, int* block_steps, int64_t* gr
  * imaginary part, each with the sources of its part) and step them as one pair;
  * phase_cos / phase_sin hold cos(k L) and sin(k L) per axis (x, y, z; entries of
  * axes without Bloch faces are ignored).  Periodic and Bloch engines run launch
- * variants 1-3 with FP32 storage, and have no adjoint. */
+ * variants 1-3 and (FP32 storage) 11, and have no adjoint. */
 typedef struct fdtd_bloch fdtd_bloch;
 int fdtd_bloch_create(fdtd_engine* re, fdtd_engine* im, const float* phase_cos, const float* phase_sin,
                       fdtd_bloch** out);
@@ -371,9 +374,9 @@ int fdtd_engine_backward_replay(fdtd_engine* h, int n_steps, int stride);
 /* Region replay (on by default): inside fdtd_engine_backward_replay, step t
  * of a T-step segment updates only the warp tasks over the design boxes grown
  * by T - t + 2 cells (the domain of dependence of the recorded design-box E:
- * one cell per step), with the scalar warp kernels; the history, and so the
- * gradient, is the full replay's bit for bit.  Applies to FP32 engines without
- * periodic / Bloch faces on launch variants 1-3 or 10; 0 replays whole steps. */
+ * one cell per step), with the scalar warp kernels or variant 11; the history, and
+ * so the gradient, is the full replay's bit for bit.  Applies to FP32 engines without
+ * periodic / Bloch faces on launch variants 1-3, 10 or 11; 0 replays whole steps. */
 int fdtd_engine_set_replay_region(fdtd_engine* h, int on);
 /* Accumulated dL/deps (absolute permittivity) of the design box of E
  * component comp (0..2), box-dense [i][j][k]. */

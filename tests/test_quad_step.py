@@ -1,0 +1,88 @@
+"""The quad-tile step kernel (launch variant 11) at the edges of its tiles: ragged
+row counts, z rows of every remainder mod 4 and of the longest length it takes,
+one-plane chunks, slabs thinner and thicker than a quad, PEC and periodic faces,
+poles, TFSF and point sources.
+
+Every tile shape gives the same bits.  Against the warp kernel (variant 2) each
+step differs by the rounding of at most three products per cell (2^-24 each), which
+add up at most linearly: 3 * 40 steps * 6e-8 = 7e-6 of the field's norm.
+"""
+import numpy as np
+import pytest
+
+from conftest import load_package
+
+pytestmark = pytest.mark.gpu
+FIELDS = ("Ex", "Ey", "Ez", "Hx", "Hy", "Hz")
+STEPS = 40
+TOL = 7e-6
+
+
+def _scene(wm, cells, pml, boundary, tfsf=False):
+    sc = wm.Scene(cells=cells, spacing=25e-9, pml_cells=pml, boundary=boundary)
+    mid = tuple(c // 2 for c in cells)
+    sc.structures.append(wm.Structure(wm.Box(tuple(m - 2 for m in mid), tuple(m + 3 for m in mid)), wm.Medium(eps_r=3.0)))
+    sc.structures.append(wm.Structure(wm.Sphere(tuple(float(m) for m in mid), 2.4), wm.Medium.lorentz(2.0, 3.0, 250e12, 20e12)))
+    pulse = wm.GaussianPulse(300e12, 100e12, delay=0.5e-15)
+    if tfsf:
+        sc.sources.append(wm.PlaneWaveTFSF((1, 0, 0), (0, 0, 1), pulse, (pml + 2,) * 3, tuple(c - pml - 2 for c in cells)))
+    else:
+        sc.sources.append(wm.PointDipole(mid, "Ez", pulse, width=25e-9))
+    return wm.compile_scene(sc, STEPS)
+
+
+def _run(wm, cs, launch):
+    solver = wm.solver.B200FDTD(cs).init_field()
+    if launch is not None:
+        solver.set_launch(*launch)
+    variant = solver.get_launch()[0]
+    solver.step_range(0, STEPS)
+    out = {n: solver.field(n).cpu().numpy() for n in FIELDS}
+    solver.close()
+    return variant, out
+
+
+@pytest.mark.parametrize("cells,pml,boundary,tfsf", [
+    ((17, 13, 12), 3, (1,) * 6, False),      # one cell beyond whole quads, thin slabs
+    ((16, 14, 15), 5, (1,) * 6, False),      # whole quads, slabs across quads
+    ((21, 30, 34), 6, (1,) * 6, True),       # TFSF faces on every axis
+    ((12, 11, 13), 0, (4,) * 6, False),      # closed box
+    ((14, 12, 29), 4, (2, 2, 2, 2, 1, 1), False),   # periodic x, y with z slabs and poles
+    ((14, 12, 18), 4, (4, 4, 2, 2, 1, 4), False),   # PEC beside periodic faces
+    ((9, 8, 511), 3, (1,) * 6, False),       # the longest row
+])
+def test_tiles_agree_with_each_other_and_with_the_warp_kernel(cells, pml, boundary, tfsf):
+    wm = load_package()
+    cs = _scene(wm, cells, min(pml, (min(cells) - 2) // 2), boundary, tfsf)
+    variant, base = _run(wm, cs, None)
+    assert variant == 11
+    top = 3 if cells[2] > 256 else 9
+    for tile in ((11, 1, 1), (11, top, 5), (11, 2, cells[0] + 1)):
+        _, got = _run(wm, cs, tile)
+        for n in FIELDS:
+            np.testing.assert_array_equal(got[n], base[n], err_msg=f"{tile} {n}")
+    _, ref = _run(wm, cs, (2, 1, 0))
+    num = sum(np.linalg.norm(base[n].astype(np.float64) - ref[n]) ** 2 / np.linalg.norm(ref[n].astype(np.float64)) ** 2 for n in FIELDS)
+    assert np.sqrt(num) <= TOL
+
+
+def test_rows_beyond_a_tile_run_another_kernel():
+    wm = load_package()
+    solver = wm.solver.B200FDTD(_scene(wm, (8, 8, 512), 2, (1,) * 6)).init_field()
+    assert solver.get_launch()[0] == 2
+    with pytest.raises(wm._lib.FdtdError):
+        solver.set_launch(11, 0, 0)
+    solver.step_range(0, 4)
+    solver.close()
+
+
+def test_a_wait_that_runs_out_is_reported():
+    wm = load_package()
+    solver = wm.solver.B200FDTD(_scene(wm, (24, 20, 18), 4, (1,) * 6)).init_field()
+    solver.set_wait_limit(0)
+    with pytest.raises(wm._lib.FdtdError) as err:
+        solver.step_range(0, 2)
+    assert "status -5" in str(err.value)
+    solver.set_wait_limit(1 << 20)
+    solver.step_range(2, 4)
+    solver.close()

@@ -45,6 +45,16 @@ __global__ void __launch_bounds__(256, 4) ade_pass_kernel(const __grid_constant_
   const unsigned mask = static_cast<unsigned>(tl.w);  // the same for every lane
   unsigned comps = 0;
   for (unsigned m = mask; m; m &= m - 1) comps |= 1u << a.poles[__ffs(m) - 1].comp;
+  // components of this row that the wrap kernel updates (except, for Ex and Ey,
+  // on a PEC z face)
+  unsigned wrapped = 0;
+  if (a.wrap_axes) {
+    const bool xw = (a.wrap_axes & 1) && (i == 0 || i == a.NX - 1), yw = (a.wrap_axes & 2) && (j == 0 || j == a.NY - 1);
+    const int pf = a.pec_bnd;
+    const bool xp = (i == 0 && (pf & 1)) || (i == a.NX - 1 && (pf & 2));
+    const bool yp = (j == 0 && (pf & 4)) || (j == a.NY - 1 && (pf & 8));
+    wrapped = (yw ? 1u : 0u) | (xw ? 2u : 0u) | ((xw || yw) && !xp && !yp ? 4u : 0u);
+  }
   bool in[kQ];
 #pragma unroll
   for (int q = 0; q < kQ; ++q) in[q] = tl.y + lane + 32 * q < tl.z;
@@ -71,6 +81,8 @@ __global__ void __launch_bounds__(256, 4) ade_pass_kernel(const __grid_constant_
     for (int q = 0; q < kQ; ++q) {
       const int k = tl.y + lane + 32 * q;
       act[q] = in[q] && k >= pt.k0 && k < pt.k1;
+      if ((wrapped >> c) & 1u)
+        act[q] = act[q] && c < 2 && ((k == 0 && (a.pec_bnd & 16)) || (k == a.NZ - 1 && (a.pec_bnd & 32)));
       drive[q] = ie[q] = pol[q] = cur[q] = 0.f;
       if (act[q]) {
         drive[q] = __ldg(pt.drive + rbase + k);

@@ -22,6 +22,7 @@
 
 #include "../../include/fdtd_b200.h"
 #include "engine.cuh"
+#include "quad_kernel.cuh"
 #include "tma_step.cuh"
 #include "adjoint.cuh"
 
@@ -329,10 +330,13 @@ constexpr int kDefaultVariant = 2;
 // prefetch into L2 (0 disables).
 constexpr int kDefaultPrefetch = 2;
 
-constexpr int kMaxVariant = 10;
+constexpr int kMaxVariant = 11;
 // The row-tile kernel (tile_kernel.cu): the default launch of FP32 engines
 // without wrapped faces.
 constexpr int kTileVariant = 10;
+// The quad-tile kernel (quad_kernel.cu): the default launch of FP32 engines
+// without PMC faces.
+constexpr int kQuadVariant = 11;
 constexpr int kTileMaxChunk = 63;  // planes per chunk of the row-tile kernel (chunk + halo plane <= 64)
 
 // z cells per lane of a launch variant (1 for the scalar kernels 1-4).
@@ -660,10 +664,16 @@ struct fdtd_engine {
   bool in_pair = false;
   int64_t plane = 0, vol = 0;
   int TY = 0, CX = 0;
+  QuadTerms qterms{};                     // injection terms of the quad-tile kernel
+  QuadShape quad{};                       // tile of the quad-tile kernel (launch variant 11)
+  unsigned char* d_quad_class = nullptr;  // its class table, sized for chunk length 1
+  int quad_key = 0;                       // chunk length the table was built for (0 = stale)
+  float *d_ztab_h = nullptr, *d_ztab_e = nullptr;
   // Fused kernel: 1..3 = register-prefetch warp kernel with a register budget
   // of up to 128 / 64 / 85 per thread; 4 = TMA-fed kernel; 5..9 = z-vectorised
   // warp kernels (vec_launcher); 10 = row-tile kernel (shared-memory row
-  // exchange, tile_kernel.cu).
+  // exchange, tile_kernel.cu); 11 = quad-tile kernel (four z cells per thread,
+  // bulk-copied planes, quad_kernel.cu).
   int variant = kDefaultVariant;
   int pf_dist = kDefaultPrefetch;
   int cur = 0;  // index of the buffer holding the current state
@@ -832,6 +842,7 @@ int background_value(fdtd_engine* h, int comp, const float* arr, float* out) {
 }
 
 int z_blocks(const fdtd_engine* h);
+int warp_chunk(const fdtd_engine* h);
 
 void fill_params(const fdtd_engine* h, StepParams& p) {
   std::memset(&p, 0, sizeof(p));
@@ -903,6 +914,10 @@ void fill_params(const fdtd_engine* h, StepParams& p) {
     if (h->desc.boundary[f] == FDTD_BND_PMC) p.pmc |= 1 << f;
   p.pec_clamp = h->lines.empty() ? 1 : 0;
   p.n_kb = z_blocks(h);
+  p.quad_class = h->d_quad_class;
+  p.fold_cx = warp_chunk(h);
+  p.ztab_h = h->d_ztab_h;
+  p.ztab_e = h->d_ztab_e;
   for (int a = 0; a < 3; ++a) {
     p.nl_lo[a] = h->nl_lo[a];
     p.nl_hi[a] = h->nl_hi[a];
@@ -927,7 +942,81 @@ int z_blocks(const fdtd_engine* h) {
   return (h->NZ + span - 1) / span;
 }
 
+// Default chunk of the warp kernel: split x until the grid holds about ten waves
+// of the 64-register variant (four 256-thread CTAs per SM on 148 SMs).  Shorter
+// chunks recompute one halo plane each, which stays cheaper than idle SMs down to
+// four planes.
+int warp_chunk(const fdtd_engine* h) {
+  if (h->desc.chunk_planes > 0) return h->desc.chunk_planes;
+  const int64_t cols = static_cast<int64_t>((h->NY + kWarpRows - 1) / kWarpRows) * ((h->NZ + kWarpOut - 1) / kWarpOut);
+  const int64_t want_chunks = std::max<int64_t>(1, (148 * 4 * 10 + cols - 1) / cols);
+  return static_cast<int>(std::max<int64_t>(4, (h->NX + want_chunks - 1) / want_chunks));
+}
+
+// Tile of the quad-tile kernel: TY rows, CX planes (ty, cx > 0 fix TY and CX).
+// Picks the smallest modelled step time; its constants come from sweeps of TY and
+// CX (B200):
+// - a plane takes a CTA `lat` when little runs beside it (65^3 with a 10-cell CPML:
+//   14 us in 3.5 plane times; 182 x 212 x 158 without: 1.5 us a plane), else its
+//   SM's share of HBM sets the time: 42 B/ns for one CTA per SM, 50 for several
+//   without CPML, which also hide most of each other's start;
+// - a chunk costs 2.5 planes beside its own (one where CTAs overlap): the halo
+//   plane and the start;
+// - without x or y slabs all CTAs take as long, and the last round of CTAs costs a
+//   whole one (257 x 257 x 193, z slabs only: 265 us at 1.9 and 7.0 rounds, 301 at
+//   2.1; 182 x 212 x 158: 56 us at TY 7, CX 10, 70 at 8, 14).  CTAs in a slab take
+//   about twice as long: the tail is 1.5 CTAs, and a single round ends with its
+//   slowest CTA (193 x 193 x 161, TY 13: 105 us at 5 planes, 133 at 22).
+void default_quad(fdtd_engine* h, int ty, int cx) {
+  const int Q = h->P / 4;
+  double best = 1e300;
+  const bool xy = h->desc.pml_lo[0] + h->desc.pml_hi[0] + h->desc.pml_lo[1] + h->desc.pml_hi[1] > 0;
+  const double lat = h->cpml ? 3000.0 : 1200.0, bytes_cell = h->cpml ? 60.0 : 48.0;
+  QuadShape s{};
+  s.nlo = std::max(1, (h->desc.pml_lo[2] + 3) / 4);
+  s.nhi = Q - (h->NZ - 1 - h->desc.pml_hi[2]) / 4;
+  if (s.nlo + s.nhi > Q) {
+    s.nlo = Q;
+    s.nhi = 0;
+  }
+  for (int TY = ty > 0 ? ty : 1; TY <= (ty > 0 ? ty : h->NY); ++TY) {
+    s.TY = TY;
+    s.threads = ((TY + 1) * Q + 31) / 32 * 32 + 32;
+    const size_t smem = quad_smem_bytes(TY, h->P, h->SZ);
+    if (s.threads > quad_max_threads(h->cpml) || smem > kQuadMaxSmem) break;
+    const int64_t rb = (h->NY + TY - 1) / TY;
+    if (ty <= 0 && TY > (h->NY + rb - 1) / rb) continue;  // a lower tile gives as many row blocks
+    const int occ = std::max(1, std::min({static_cast<int>(kQuadMaxSmem / (smem + 1024)),
+                                          65536 / (quad_regs(h->cpml) * s.threads), 2048 / s.threads, 32}));
+    for (int C = 1; C <= h->NX; ++C) {
+      const int CX = cx > 0 ? cx : (h->NX + C - 1) / C;
+      if (cx <= 0 && C > 1 && CX == (h->NX + C - 2) / (C - 1)) continue;
+      const int64_t chunks = (h->NX + CX - 1) / CX;
+      const double blocks = static_cast<double>(rb * chunks);
+      const double resident = std::min<double>(occ, std::ceil(blocks / 148));
+      const bool one = resident < 2.0 || h->cpml;
+      const double plane = std::max(lat, resident * (TY * bytes_cell + 36.0) * h->P / (one ? 42.0 : 50.0));
+      const double cta = (CX + (chunks > 1 ? 1.0 : 0.0) + (one ? 1.5 : 0.0)) * plane;
+      const double waves = blocks / (148.0 * occ);
+      const double cost = cta * (!xy ? std::ceil(waves) : waves <= 1.0 ? 2.0 : waves + 1.5);
+      if (cost < best) {
+        best = cost;
+        h->quad = s;
+        h->TY = TY;
+        h->CX = CX;
+      }
+      if (cx > 0) break;
+    }
+  }
+}
+
 void default_tiles(fdtd_engine* h) {
+  if (h->variant == kQuadVariant) {
+    default_quad(h, h->desc.tile_rows, h->desc.chunk_planes);
+    if (h->quad.threads > 0) return;
+    default_quad(h, 0, h->desc.chunk_planes);  // the caller's tile rows do not fit
+    return;
+  }
   h->TY = 1;
   int CX = h->desc.chunk_planes;
   if (CX <= 0 && variant_v(h->variant) > 1) {
@@ -947,20 +1036,20 @@ void default_tiles(fdtd_engine* h) {
     const int64_t want_chunks = std::max<int64_t>(1, (148 * 3 * 13 + cols - 1) / cols);
     CX = static_cast<int>(std::min<int64_t>(kTileMaxChunk, std::max<int64_t>(12, (h->NX + want_chunks - 1) / want_chunks)));
   }
-  if (CX <= 0) {
-    // Split x into chunks until the grid holds about ten waves of the
-    // 64-register variant (four 256-thread CTAs per SM on 148 SMs).  Shorter
-    // chunks recompute one halo plane each, which stays cheaper than idle SMs
-    // down to four planes.
-    const int64_t cols = static_cast<int64_t>((h->NY + kWarpRows - 1) / kWarpRows) * ((h->NZ + kWarpOut - 1) / kWarpOut);
-    const int64_t want_chunks = std::max<int64_t>(1, (148 * 4 * 10 + cols - 1) / cols);
-    CX = static_cast<int>(std::max<int64_t>(4, (h->NX + want_chunks - 1) / want_chunks));
-  }
+  if (CX <= 0) CX = warp_chunk(h);
   h->CX = CX;
 }
 
-dim3 step_grid(const fdtd_engine* h) {
+bool quad_runs(const fdtd_engine* h);
+
+// Task grid of the warp kernel (and of the other kernels with its layout).
+dim3 warp_grid(const fdtd_engine* h) {
   return dim3((h->NY + kWarpRows - 1) / kWarpRows, z_blocks(h), (h->NX + h->CX - 1) / h->CX);
+}
+
+dim3 step_grid(const fdtd_engine* h) {
+  if (!quad_runs(h)) return warp_grid(h);
+  return dim3((h->NY + h->TY - 1) / h->TY, 1, (h->NX + h->CX - 1) / h->CX);
 }
 
 // Read (and clear) the device status word after the stream has drained.
@@ -984,9 +1073,17 @@ bool has_coef(const fdtd_engine* h) {
   return false;
 }
 
-// Build the per-warp class table for the current launch shape if it is stale.
+// Build the class table of the current launch shape if it is stale.
 int ensure_classified(fdtd_engine* h, const StepParams& p) {
-  const dim3 grid = step_grid(h);
+  if (quad_runs(h)) {
+    if (has_coef(h) && h->quad_key != h->CX) {
+      const int err = launch_quad_classify(p, static_cast<int>(step_grid(h).z), h->d_quad_class, h->stream);
+      if (err != 0) return cuda_fail(static_cast<cudaError_t>(err), "quad_classify_kernel launch");
+      h->quad_key = h->CX;
+    }
+    return 0;
+  }
+  const dim3 grid = warp_grid(h);
   const int V = variant_v(h->variant);
   const int key = h->CX * 8 + V;
   if ((h->cpml || has_coef(h)) && h->class_key != key) {
@@ -1003,7 +1100,15 @@ int ensure_classified(fdtd_engine* h, const StepParams& p) {
 // on FP32 storage with the scalar step kernels and no wrapped face.
 bool ade_pass_active(const fdtd_engine* h) {
   return h->ade_pass && h->n_ade_tiles > 0 && h->poles.size() <= static_cast<size_t>(kAdeMaxPoles) &&
-         h->storage == kStoreF32 && !h->wrap && ((h->variant >= 1 && h->variant <= 3) || h->variant == kTileVariant);
+         h->storage == kStoreF32 &&
+         ((!h->wrap && ((h->variant >= 1 && h->variant <= 3) || h->variant == kTileVariant)) || h->variant == kQuadVariant);
+}
+
+// The quad-tile kernel has no pole code: as for the row-tile kernel, the
+// 64-register warp kernel runs where the ADE pass cannot take the poles.
+bool quad_runs(const fdtd_engine* h) {
+  return h->variant == kQuadVariant && h->storage == kStoreF32 && !h->pmc && h->P <= kQuadMaxPitch &&
+         h->terms.size() <= static_cast<size_t>(kQuadMaxTerms) && (h->poles.empty() || ade_pass_active(h));
 }
 
 // The row-tile kernel has no pole code: with poles that the ADE pass cannot
@@ -1117,8 +1222,18 @@ int launch_step(fdtd_engine* h, int n, int slot, const int* region = nullptr) {
   }
   StepParams p;
   fill_params(h, p);
+  const bool quad = quad_runs(h);
   dim3 grid = step_grid(h);
-  if (region) {
+  if (region && quad) {
+    // the quad-tile kernel splits rows and planes only
+    const unsigned rb0 = static_cast<unsigned>(region[2] / h->TY), ch0 = static_cast<unsigned>(region[0] / h->CX);
+    const unsigned rb1 = std::min<unsigned>(grid.x, static_cast<unsigned>((region[3] + h->TY - 1) / h->TY));
+    const unsigned ch1 = std::min<unsigned>(grid.z, static_cast<unsigned>((region[1] + h->CX - 1) / h->CX));
+    if (rb1 <= rb0 || ch1 <= ch0) return fail(FDTD_ERR_INVALID_ARG, "empty step region");
+    p.rb0 = static_cast<int>(rb0);
+    p.ch0 = static_cast<int>(ch0);
+    grid = dim3(rb1 - rb0, grid.y, ch1 - ch0);
+  } else if (region) {
     const unsigned rb0 = static_cast<unsigned>(region[2] / kWarpRows), kb0 = static_cast<unsigned>(region[4] / kWarpOut);
     const unsigned ch0 = static_cast<unsigned>(region[0] / h->CX);
     const unsigned rb1 = std::min<unsigned>(grid.x, static_cast<unsigned>((region[3] + kWarpRows - 1) / kWarpRows));
@@ -1149,6 +1264,9 @@ int launch_step(fdtd_engine* h, int n, int slot, const int* region = nullptr) {
   if (h->storage != kStoreF32) {
     const int err = launch_step_reduced(p, n, grid, h->cpml, coef, h->uniform_grid, h->stream);
     if (err != 0) return cuda_fail(static_cast<cudaError_t>(err), "warp_step_kernel_rs launch");
+  } else if (quad) {
+    const int err = launch_quad_step(p, h->qterms, h->quad, n, grid, coef, h->uniform_grid, h->stream);
+    if (err != 0) return cuda_fail(static_cast<cudaError_t>(err), "quad_step_kernel launch");
   } else if (!region && tile_runs(h)) {
     // the row-tile kernel, then (scenes with CPML) the warp kernel over the
     // CTAs that meet a slab, which the row-tile kernel leaves alone
@@ -1178,8 +1296,8 @@ int launch_step(fdtd_engine* h, int n, int slot, const int* region = nullptr) {
   do {                                                                                           \
     if (h->variant == 4)                                                                          \
       tma_step_kernel<CPML, COEF, UNI><<<grid, kTmaThreads, tma_smem_bytes(), h->stream>>>(p, h->maps[h->cur], n); \
-    else if ((h->variant == 2 || h->variant == kTileVariant) && ade_pass) warp_step_kernel<CPML, COEF, UNI, 4, false><<<grid, block, 0, h->stream>>>(p, n, slot); \
-    else if (h->variant == 2 || h->variant == kTileVariant) warp_step_kernel<CPML, COEF, UNI, 4, true><<<grid, block, 0, h->stream>>>(p, n, slot); \
+    else if ((h->variant == 2 || h->variant >= kTileVariant) && ade_pass) warp_step_kernel<CPML, COEF, UNI, 4, false><<<grid, block, 0, h->stream>>>(p, n, slot); \
+    else if (h->variant == 2 || h->variant >= kTileVariant) warp_step_kernel<CPML, COEF, UNI, 4, true><<<grid, block, 0, h->stream>>>(p, n, slot); \
     else if (h->variant == 3 && ade_pass) warp_step_kernel<CPML, COEF, UNI, 3, false><<<grid, block, 0, h->stream>>>(p, n, slot); \
     else if (h->variant == 3) warp_step_kernel<CPML, COEF, UNI, 3, true><<<grid, block, 0, h->stream>>>(p, n, slot); \
     else warp_step_kernel<CPML, COEF, UNI, 1, true><<<grid, block, 0, h->stream>>>(p, n, slot);            \
@@ -1484,12 +1602,11 @@ int fdtd_engine_create(const fdtd_grid_desc* desc, void* stream, fdtd_engine** o
     fdtd_engine_destroy(h);
     return rc;
   }
-  // The row-tile kernel is the default where it measured fastest: FP32 scenes
-  // without CPML or wrapped faces (256^3 vacuum: 0.201 against 0.253 ms).  With
-  // CPML the slab CTAs run in the warp kernel either way and the hybrid launch
-  // measured no faster (CPML vacuum 0.389 against 0.393 ms, the dispersive
-  // workload 0.520 against 0.509 ms), so those engines keep variant 2.
-  if (!h->wrap && !h->cpml && !h->pmc) h->variant = kTileVariant;
+  // The quad-tile kernel runs where a row fits its CTA and no face is PMC.  Beside
+  // it stay the row-tile kernel (longer rows without CPML or wrapped faces) and
+  // the warp kernel.
+  if (!h->pmc && h->P <= kQuadMaxPitch) h->variant = kQuadVariant;
+  else if (!h->wrap && !h->cpml && !h->pmc) h->variant = kTileVariant;
   default_tiles(h);
   *out = h;
   return 0;
@@ -1516,6 +1633,7 @@ int fdtd_engine_destroy(fdtd_engine* h) {
   for (int* p : h->index_bufs) cudaFree(p);
   cudaFree(h->d_flush);
   cudaFree(h->d_warp_class);
+  cudaFree(h->d_quad_class);
   for (float* p : h->adj.bufs) cudaFree(p);
   cudaFree(h->d_status);
   cudaFree(h->d_base);
@@ -1575,7 +1693,10 @@ int fdtd_engine_set_storage(fdtd_engine* h, int kind, const float* scales) {
   }
   for (int c = 0; c < 6; ++c) h->fscale[c] = scales ? scales[c] : 1.0f;
   h->scales_set = scales != nullptr;
-  if (kind != kStoreF32) h->variant = 2;
+  if (kind != kStoreF32) {
+    h->variant = 2;
+    default_tiles(h);
+  }
   return 0;
 }
 
@@ -2178,8 +2299,8 @@ int fdtd_engine_finalize(fdtd_engine* h) {
     if (!h->poles.empty()) {
       if (!h->ade_pass || h->poles.size() > static_cast<size_t>(kAdeMaxPoles))
         return fail(FDTD_ERR_UNSUPPORTED, "nonlinear media with poles need the ADE pass (at most 32 pole components)");
-      if (h->variant >= 4 && h->variant != kTileVariant)
-        return fail(FDTD_ERR_UNSUPPORTED, "nonlinear media with poles run launch variants 1-3 and 10");
+      if (h->variant >= 4 && h->variant < kTileVariant)
+        return fail(FDTD_ERR_UNSUPPORTED, "nonlinear media with poles run launch variants 1-3, 10 and 11");
     }
     const int64_t n = static_cast<int64_t>(h->nl_cells_h.size() / 4);
     CUDA_TRY(cudaMalloc(&h->d_nl_cells, sizeof(int4) * n));
@@ -2221,6 +2342,18 @@ int fdtd_engine_finalize(fdtd_engine* h) {
     h->d_pole_ptr = const_cast<int*>(dp);
     h->d_pole_ids = const_cast<int*>(di);
   }
+  h->qterms.n = static_cast<int>(std::min<size_t>(h->terms.size(), kQuadMaxTerms));
+  std::copy_n(h->terms.begin(), h->qterms.n, h->qterms.t);
+  h->qterms.h_bits = 0;
+  for (int b = 0; b < h->qterms.n; ++b)
+    if (h->qterms.t[b].comp >= 3) h->qterms.h_bits |= 1u << b;
+  if (h->variant == kQuadVariant && (h->poles.size() > static_cast<size_t>(kAdeMaxPoles) ||
+                                     h->terms.size() > static_cast<size_t>(kQuadMaxTerms))) {
+    // more poles than the ADE pass takes, or more injection terms than the
+    // quad-tile kernel's table: the warp kernel runs
+    h->variant = kDefaultVariant;
+    default_tiles(h);
+  }
   if (!h->poles.empty() && h->poles.size() <= static_cast<size_t>(kAdeMaxPoles)) {
     // ADE pass: the pole table, and tiles over the z range of each (i, j) row
     // covered by any pole box, cut into 32 * kAdeCellsPerLane-cell pieces (one
@@ -2231,6 +2364,12 @@ int fdtd_engine_finalize(fdtd_engine* h) {
     a.NX = h->NX;
     a.NZ = h->NZ;
     a.pec_faces = 0;
+    a.wrap_axes = 0;
+    a.pec_bnd = 0;
+    for (int f = 0; f < 6; ++f)
+      if (h->desc.boundary[f] == FDTD_BND_PEC) a.pec_bnd |= 1 << f;
+    for (int ax = 0; ax < 2; ++ax)
+      if (h->desc.boundary[2 * ax] == FDTD_BND_PERIODIC || h->desc.boundary[2 * ax] == FDTD_BND_BLOCH) a.wrap_axes |= 1 << ax;
     for (int c = 0; c < 3; ++c) a.nl_curl[c] = h->nl_general >= 0 ? h->ecoef[c][1] : nullptr;
     if (h->lines.empty())
       for (int f = 0; f < 6; ++f)
@@ -2368,6 +2507,20 @@ int fdtd_engine_finalize(fdtd_engine* h) {
     const int64_t kblocks = (h->NZ + kWarpOut - 1) / kWarpOut;
     CUDA_TRY(cudaMalloc(&h->d_warp_class, static_cast<size_t>(h->NX) * kblocks * h->NY));
     h->class_key = 0;
+    h->quad_key = 0;
+    if (h->storage == kStoreF32 && has_coef(h))
+      CUDA_TRY(cudaMalloc(&h->d_quad_class, static_cast<size_t>(h->NX) * h->NY * (h->P / 4)));
+    if (h->storage == kStoreF32) {
+      rc = dev_alloc(h, &h->d_ztab_h, 4 * static_cast<size_t>(h->P));
+      if (!rc) rc = dev_alloc(h, &h->d_ztab_e, 4 * static_cast<size_t>(h->P));
+      if (rc) return rc;
+      const int lo = h->desc.pml_lo[2], hi = h->desc.pml_hi[2];
+      int err = launch_quad_ztable(h->hb[2], h->hc[2], h->hik[2], h->inv_h[2], h->NZ - 1, lo, hi, h->P, h->d_ztab_h,
+                                   h->stream);
+      if (err == 0)
+        err = launch_quad_ztable(h->eb[2], h->ec[2], h->eik[2], h->inv_e[2], h->NZ, lo, hi, h->P, h->d_ztab_e, h->stream);
+      if (err != 0) return cuda_fail(static_cast<cudaError_t>(err), "quad_ztable_kernel launch");
+    }
     CUDA_TRY(cudaMalloc(&h->d_status, sizeof(int)));
     CUDA_TRY(cudaMemsetAsync(h->d_status, 0, sizeof(int), h->stream));
     CUDA_TRY(cudaMalloc(&h->d_base, sizeof(int)));
@@ -2608,14 +2761,22 @@ int fdtd_engine_autotune(fdtd_engine* h, int* tile_rows, int* chunk_planes) {
   const int cxs[] = {4, 6, 8, 12, 16, 24, 32, 48};
   float best = 1e30f;
   int best_ty = 1, best_cx = h->CX, best_var = h->variant;
-  for (int var = 1; var <= kMaxVariant; ++var) {
+  // an engine that runs the quad-tile kernel tunes its tile: every tile gives the
+  // same bits, which the other kernels (slower wherever it runs) do not
+  const int first = quad_runs(h) ? kQuadVariant : 1;
+  for (int var = first; var <= kMaxVariant; ++var) {
     if (var == 4 && !h->tma_ready) continue;
     if (h->storage != kStoreF32 && var != 2) continue;  // reduced storage: the 64-register kernel only
-    if ((h->wrap || h->pmc) && var > 3) continue;        // wrap and PMC faces: the scalar warp kernels only
-    if (h->nl_n > 0 && !h->poles.empty() && var > 3 && var != kTileVariant) continue;  // nonlinear poles: the ADE pass
+    // wrap faces: the scalar warp kernels and the quad-tile kernel; PMC faces: the former only
+    if (h->wrap && var > 3 && var != kQuadVariant) continue;
+    if (h->pmc && var > 3) continue;
+    if (var == kQuadVariant && (h->P > kQuadMaxPitch || h->terms.size() > static_cast<size_t>(kQuadMaxTerms))) continue;
+    if (h->nl_n > 0 && !h->poles.empty() && var > 3 && var < kTileVariant) continue;  // nonlinear poles: the ADE pass
     for (int cx : cxs) {
       if (cx > 2 * h->NX) continue;
       h->variant = var;
+      h->TY = 1;
+      if (var == kQuadVariant) default_quad(h, 0, cx);
       h->CX = cx;
       const int reps = 3;
       rc = launch_step(h, 0, -1);
@@ -2632,13 +2793,15 @@ int fdtd_engine_autotune(fdtd_engine* h, int* tile_rows, int* chunk_planes) {
       if (ms < best) {
         best = ms;
         best_cx = cx;
+        best_ty = h->TY;
         best_var = var;
       }
     }
   }
-  h->TY = best_ty;
   h->CX = best_cx;
   h->variant = best_var;
+  if (best_var == kQuadVariant) default_quad(h, best_ty, best_cx);
+  h->TY = best_ty;
   rc = fdtd_engine_checkpoint_load(h, slot);
   if (rc) return rc;
   cudaFree(h->checkpoints[slot].store);
@@ -2673,15 +2836,32 @@ int fdtd_engine_time_kernel(fdtd_engine* h, int n, int reps, float* ms) {
 int fdtd_engine_set_launch(fdtd_engine* h, int variant, int tile_rows, int chunk_planes) {
   if (!h || variant < 1 || variant > kMaxVariant || tile_rows < 0 || chunk_planes < 0)
     return fail(FDTD_ERR_INVALID_ARG, "bad launch configuration");
-  (void)tile_rows;  // the warp-granular kernels have no tile height
   if (h->storage != kStoreF32 && variant != 2)
     return fail(FDTD_ERR_UNSUPPORTED, "reduced field storage runs launch variant 2 only");
-  if (h->wrap && variant > 3)
-    return fail(FDTD_ERR_UNSUPPORTED, "periodic and Bloch faces run launch variants 1-3 only");
+  if (h->wrap && variant > 3 && variant != kQuadVariant)
+    return fail(FDTD_ERR_UNSUPPORTED, "periodic and Bloch faces run launch variants 1-3 and 11 only");
   if (h->pmc && variant > 3) return fail(FDTD_ERR_UNSUPPORTED, "PMC faces run launch variants 1-3 only");
-  if (h->nl_general >= 0 && !h->poles.empty() && variant > 3 && variant != kTileVariant)
-    return fail(FDTD_ERR_UNSUPPORTED, "nonlinear media with poles run launch variants 1-3 and 10");
+  if (variant == kQuadVariant && (h->P > kQuadMaxPitch || h->terms.size() > static_cast<size_t>(kQuadMaxTerms)))
+    return fail(FDTD_ERR_UNSUPPORTED, "the quad-tile kernel takes up to 512 z nodes and 24 injection terms");
+  if (h->nl_general >= 0 && !h->poles.empty() && variant > 3 && variant < kTileVariant)
+    return fail(FDTD_ERR_UNSUPPORTED, "nonlinear media with poles run launch variants 1-3, 10 and 11");
+  if (variant == kQuadVariant) {
+    // the only tile with rows: an explicit height has to fit a CTA
+    const QuadShape keep = h->quad;
+    const int TY0 = h->TY, CX0 = h->CX;
+    h->quad = QuadShape{};
+    default_quad(h, tile_rows > 0 ? tile_rows : h->desc.tile_rows, chunk_planes > 0 ? chunk_planes : h->desc.chunk_planes);
+    if (h->quad.threads == 0) {
+      h->quad = keep;
+      h->TY = TY0;
+      h->CX = CX0;
+      return fail(FDTD_ERR_INVALID_ARG, "tile_rows does not fit a CTA of the quad-tile kernel");
+    }
+    h->variant = variant;
+    return 0;
+  }
   h->variant = variant;
+  h->TY = 1;
   if (chunk_planes > 0) h->CX = chunk_planes;
   else default_tiles(h);
   // the row-tile kernel gathers its chunk's plane bits into 64-bit masks
@@ -2978,7 +3158,7 @@ int fdtd_engine_backward_replay(fdtd_engine* h, int n_steps, int stride) {
   // (same kernel bodies per task, bit for bit).  Cells outside the region
   // keep stale values, which nothing reads before the next checkpoint load.
   const bool region_ok = h->replay_region && design && h->storage == kStoreF32 && !h->wrap &&
-                         ((h->variant >= 1 && h->variant <= 3) || h->variant == kTileVariant);
+                         ((h->variant >= 1 && h->variant <= 3) || h->variant >= kTileVariant);
   int dbox[6] = {INT_MAX, -1, INT_MAX, -1, INT_MAX, -1};
   for (int c = 0; c < 3; ++c) {
     const DesignBox& d = a.q.design[c];
@@ -3146,7 +3326,7 @@ int fdtd_engine_info(fdtd_engine* h, int* tile_rows, int* chunk_planes, int* gri
   const dim3 g = step_grid(h);
   if (grid_x) *grid_x = static_cast<int>(g.x);
   if (grid_y) *grid_y = static_cast<int>(g.y * g.z);
-  if (block) *block = tile_runs(h) ? tile_block_threads() : kWarpRows * 32;
+  if (block) *block = quad_runs(h) ? h->quad.threads : tile_runs(h) ? tile_block_threads() : kWarpRows * 32;
   if (launches) *launches = h->launches;
   return 0;
 }
@@ -3476,7 +3656,9 @@ int fdtd_bloch_create(fdtd_engine* re, fdtd_engine* im, const float* phase_cos, 
   for (int f = 0; f < 6; ++f) same = same && a.boundary[f] == b.boundary[f];
   for (int x = 0; x < 3; ++x) same = same && a.pml_lo[x] == b.pml_lo[x] && a.pml_hi[x] == b.pml_hi[x];
   if (!same) return fail(FDTD_ERR_INVALID_ARG, "the two channels need the same grid, boundaries, stream and sample block");
-  if (re->variant > 3 || im->variant > 3) return fail(FDTD_ERR_UNSUPPORTED, "Bloch pairs run launch variants 1-3");
+  for (const fdtd_engine* h : {re, im})
+    if (h->variant > 3 && h->variant != kQuadVariant)
+      return fail(FDTD_ERR_UNSUPPORTED, "Bloch pairs run launch variants 1-3 and 11");
   fdtd_bloch* p = new fdtd_bloch();
   p->re = re;
   p->im = im;

@@ -161,6 +161,13 @@ struct StepParams {
   // starting at (rb0, kb0, ch0) of the full task grid, whose z-block count is
   // n_kb (the class table's layout); 0, 0, 0 and gridDim.y for a full launch.
   int rb0, kb0, ch0, n_kb;
+  // Quad-tile kernel (quad_kernel.cu): class bits per (chunk, row, four-cell z
+  // group), and the H and E z tables ([4][P]: b, c, 1/kappa, neutral outside
+  // the slabs, and the inverse spacing).
+  const unsigned char* quad_class;
+  int fold_cx;  // planes of an x block of its rounding rule (the warp kernel's default chunk)
+  const float* ztab_h;
+  const float* ztab_e;
 };
 
 // A warp task needs the CPML code (some cell of its footprint lies in a slab)
@@ -202,6 +209,10 @@ struct AdeParams {
   // PEC faces (bit f for face f) whose tangential E stays zero after the pass
   // (StepParams::pec_clamp), and the grid extents the face test needs
   int pec_faces, NX, NZ;
+  // wrapped axes (bit 0 x, bit 1 y) and PEC faces (bit f): the E cells on a
+  // wrapped face that touch no PEC face (edge mode kModeDeferred), and their
+  // poles, belong to the wrap kernel
+  int wrap_axes, pec_bnd;
   // Scenes with an instantaneous nonlinearity subtract J times the E curl
   // coefficient of this step (dt 1) instead of dt J / eps
   // (witwin/maxwell/fdtd/runtime/materials.py:751-773); nullptr otherwise.
