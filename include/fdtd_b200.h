@@ -207,6 +207,13 @@ int fdtd_engine_set_dft_windows(fdtd_engine* h, int n_freq, const double* omega,
 /* Read the accumulated DFT: re/im device arrays of n_freq * n_samples floats,
  * [freq][slot] order, unscaled (scale 2/sum(window) is applied by the caller). */
 int fdtd_engine_read_dft(fdtd_engine* h, float* re, float* im);
+/* Scaled complex spectra of n_items (sample region, frequency) pairs, region in the
+ * order of fdtd_engine_add_sample_region: block b holds the region's cells, one
+ * after another in `out` (device, interleaved re, im), times scale[freq[b]] (host,
+ * one per DFT frequency).  imag: the imaginary channel of a Bloch pair,
+ * or NULL.  One launch on the engine's stream; nothing waits for it. */
+int fdtd_engine_read_spectra(fdtd_engine* h, fdtd_engine* imag, int n_items, const int* region, const int* freq,
+                             const float* scale, float* out);
 
 /* Freeze the scene description and build device tables.  Must precede stepping. */
 int fdtd_engine_finalize(fdtd_engine* h);

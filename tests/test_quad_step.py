@@ -86,3 +86,36 @@ def test_a_wait_that_runs_out_is_reported():
     solver.set_wait_limit(1 << 20)
     solver.step_range(2, 4)
     solver.close()
+
+
+@pytest.mark.parametrize("bloch", [False, True])
+def test_spectra_equal_the_scaled_accumulators(bloch):
+    """monitor_results against raw_dft, scaled here: the same products, so the same
+    bits.  Monitors of other frequencies, a one-cell monitor and a whole plane."""
+    import torch
+
+    wm = load_package()
+    sc = wm.Scene(cells=(18, 14, 20), spacing=25e-9, pml_cells=4, boundary=(3, 3, 2, 2, 1, 1) if bloch else (1,) * 6,
+                  bloch_k=(2e6, 0.0, 0.0) if bloch else (0.0, 0.0, 0.0))
+    sc.sources.append(wm.PointDipole((9, 7, 10), "Ex", wm.GaussianPulse(300e12, 100e12, delay=0.5e-15), width=25e-9))
+    sc.monitors.append(wm.PlaneMonitor("plane", 2, 8, frequencies=(250e12, 300e12, 350e12)))
+    sc.monitors.append(wm.PointMonitor("point", (8, 6, 9), frequencies=(350e12, 250e12)))
+    cs = wm.compile_scene(sc, STEPS)
+    solver = wm.solver.B200FDTD(cs).init_field()
+    solver.step_range(0, STEPS)
+    got, host = solver.monitor_results(), solver.monitor_results(host=True)
+    re, im = solver.raw_dft()
+    if bloch:
+        rb, ib = solver.raw_dft(imag=True)
+        re, im = re - ib, im + rb
+    scale = wm.scene.window_scales(cs.window, STEPS, len(cs.frequencies)).astype(np.float32)
+    for reg, base in zip(cs.regions, solver.region_base):
+        b = reg.box
+        shape = (b[1] - b[0], b[3] - b[2], b[5] - b[4])
+        for n, f in enumerate(cs.monitor_frequencies[reg.monitor]):
+            at = cs.frequencies.index(f)
+            want = torch.complex(re[at] * float(scale[at]), im[at] * float(scale[at]))[base:base + int(np.prod(shape))]
+            v = got[reg.monitor][reg.component][n]
+            assert torch.equal(v, want.reshape(shape))
+            assert torch.equal(host[reg.monitor][reg.component][n], v.cpu())
+    solver.close()

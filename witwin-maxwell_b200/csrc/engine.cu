@@ -318,6 +318,36 @@ __global__ void dft_flush_kernel(const float* samples, int64_t n_samples, int cn
   }
 }
 
+// Scaled complex spectra of every (region, frequency) pair asked for, in one
+// launch: item b covers slots [src, src + count) of frequency freq and writes
+// out[dst ..].  A Bloch field F = A + iB has DFT(F) = DFT(A) + i DFT(B).  The work
+// is 16 bytes a value; in place of it stood a dozen small launches and table
+// uploads per region (32 regions of 16 frequencies at 131^3: 3.8 ms of host time).
+struct SpectraItem {
+  int64_t src, count, dst;
+  int64_t freq;
+};
+constexpr int kMaxFreq = 256;  // as fdtd_engine_set_dft
+struct SpectraScale {
+  float s[kMaxFreq];
+};
+__global__ void __launch_bounds__(256) spectra_kernel(const SpectraItem* items, const float* re, const float* im,
+                                                      const float* re_b, const float* im_b, int64_t n_samples,
+                                                      const __grid_constant__ SpectraScale scale, float2* out) {
+  const SpectraItem it = items[blockIdx.y];
+  const float sc = scale.s[it.freq];
+  const int64_t base = it.freq * n_samples + it.src;
+  for (int64_t x = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; x < it.count;
+       x += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    float a = re[base + x], b = im[base + x];
+    if (re_b) {
+      a -= im_b[base + x];
+      b += re_b[base + x];
+    }
+    out[it.dst + x] = make_float2(a * sc, b * sc);
+  }
+}
+
 }  // namespace
 
 struct DevBuf {
@@ -738,6 +768,9 @@ struct fdtd_engine {
   float2* w_e = nullptr;
   float2* w_h = nullptr;
   float *acc_re = nullptr, *acc_im = nullptr, *cmp_re = nullptr, *cmp_im = nullptr;
+  // Work list of the last spectra read (fdtd_engine_read_spectra) and its key
+  SpectraItem* d_spectra = nullptr;
+  std::vector<int> spectra_key;
   bool finalized = false;
   int64_t launches = 0;
   float last_ms = 0.0f;
@@ -1644,6 +1677,7 @@ int fdtd_engine_destroy(fdtd_engine* h) {
   cudaFree(h->acc_im);
   cudaFree(h->cmp_re);
   cudaFree(h->cmp_im);
+  cudaFree(h->d_spectra);
   if (h->aux) cudaStreamSynchronize(h->aux);
   for (cudaEvent_t e : {h->ev_fork, h->ev_join, h->ev_gat[0], h->ev_gat[1]})
     if (e) cudaEventDestroy(e);
@@ -2666,6 +2700,49 @@ int fdtd_engine_read_dft(fdtd_engine* h, float* re, float* im) {
   const size_t bytes = sizeof(float) * static_cast<size_t>(h->n_freq) * h->n_samples;
   CUDA_TRY(cudaMemcpyAsync(re, h->acc_re, bytes, cudaMemcpyDefault, h->stream));
   CUDA_TRY(cudaMemcpyAsync(im, h->acc_im, bytes, cudaMemcpyDefault, h->stream));
+  return 0;
+}
+
+int fdtd_engine_read_spectra(fdtd_engine* h, fdtd_engine* imag, int n_items, const int* region, const int* freq,
+                             const float* scale, float* out) {
+  if (!h || n_items < 1 || !region || !freq || !scale || !out)
+    return fail(FDTD_ERR_INVALID_ARG, "bad spectra read arguments");
+  if (!h->acc_re || (imag && !imag->acc_re)) return fail(FDTD_ERR_STATE, "no DFT accumulators");
+  if (imag && (imag->n_freq != h->n_freq || imag->n_samples != h->n_samples || imag->stream != h->stream))
+    return fail(FDTD_ERR_INVALID_ARG, "the two channels need the same monitors, frequencies and stream");
+  for (int b = 0; b < n_items; ++b)
+    if (region[b] < 0 || region[b] >= static_cast<int>(h->regions.size()) || freq[b] < 0 || freq[b] >= h->n_freq)
+      return fail(FDTD_ERR_INVALID_ARG, "no such sample region or frequency");
+  int rc = flush_samples(h);
+  if (!rc && imag) rc = flush_samples(imag);
+  if (rc) return rc;
+  std::vector<int> key(region, region + n_items);
+  key.insert(key.end(), freq, freq + n_items);
+  if (key != h->spectra_key) {
+    std::vector<SpectraItem> items(n_items);
+    int64_t dst = 0;
+    for (int b = 0; b < n_items; ++b) {
+      const SampleRegion& r = h->regions[region[b]];
+      const int64_t count = static_cast<int64_t>(r.i1 - r.i0) * (r.j1 - r.j0) * (r.k1 - r.k0);
+      items[b] = {r.base, count, dst, freq[b]};
+      dst += count;
+    }
+    h->spectra_key.clear();
+    rc = upload_vec(h, &h->d_spectra, items);
+    if (rc) return rc;
+    CUDA_TRY(cudaStreamSynchronize(h->stream));  // the list is a local
+    h->spectra_key = key;
+  }
+  SpectraScale sc{};
+  std::copy_n(scale, h->n_freq, sc.s);
+  const unsigned gx = static_cast<unsigned>(std::min<int64_t>((h->max_region + 255) / 256, 1024));
+  for (int b = 0; b < n_items; b += 65535) {  // the grid's y limit
+    spectra_kernel<<<dim3(std::max(gx, 1u), std::min(n_items - b, 65535)), 256, 0, h->stream>>>(
+        h->d_spectra + b, h->acc_re, h->acc_im, imag ? imag->acc_re : nullptr, imag ? imag->acc_im : nullptr, h->n_samples,
+        sc, reinterpret_cast<float2*>(out));
+    CUDA_TRY(cudaGetLastError());
+    ++h->launches;
+  }
   return 0;
 }
 
