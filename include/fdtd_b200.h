@@ -49,6 +49,10 @@ extern "C" {
 /* Last error message of the calling thread (engine-independent). */
 const char* fdtd_last_error(void);
 /* Library version string. */
+/* The engines of a device take their arrays from one memory pool, which keeps up to
+ * 4 GiB of what destroyed engines gave back.  This returns all but keep_bytes of the
+ * unused memory to the current device (it waits for the device first). */
+int fdtd_release_memory(uint64_t keep_bytes);
 const char* fdtd_version(void);
 
 /* ------------------------------------------------------------------------ */

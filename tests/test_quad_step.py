@@ -119,3 +119,22 @@ def test_spectra_equal_the_scaled_accumulators(bloch):
             assert torch.equal(v, want.reshape(shape))
             assert torch.equal(host[reg.monitor][reg.component][n], v.cpu())
     solver.close()
+
+
+def test_released_memory_goes_back_to_the_device():
+    """A closed solver's arrays stay in the pool (a second one of the same scene takes
+    them from there) until they are given back."""
+    import torch
+
+    wm = load_package()
+    cs = wm.compile_scene(wm.Scene(cells=(96, 96, 96), spacing=25e-9, pml_cells=8), 4)
+    wm.solver.release_memory()
+    free = torch.cuda.mem_get_info()[0]
+    for _ in range(2):
+        solver = wm.solver.B200FDTD(cs).init_field()
+        solver.step_range(0, 2)
+        assert float(solver.field("Ez").abs().max()) == 0.0  # pooled memory starts at zero too
+        solver.set_field("Ez", torch.ones(wm.scene.component_shape("Ez", cs.nodes), device="cuda"))
+        solver.close()
+    wm.solver.release_memory()
+    assert torch.cuda.mem_get_info()[0] >= free - (64 << 20)  # torch's own cache: three 3.5 MB fields

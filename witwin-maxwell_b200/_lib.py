@@ -73,6 +73,7 @@ _SIGNATURES = {
     "fdtd_engine_set_dft": ([_vp, _i, ctypes.POINTER(_d), _i, ctypes.POINTER(_d)], _i),
     "fdtd_engine_set_dft_windows": ([_vp, _i, ctypes.POINTER(_d), _i, ctypes.POINTER(_d)], _i),
     "fdtd_engine_read_dft": ([_vp, _vp, _vp], _i),
+    "fdtd_release_memory": ([ctypes.c_uint64], _i),
     "fdtd_engine_read_spectra": ([_vp, _vp, _i, _vp, _vp, _vp, _vp], _i),
     "fdtd_engine_finalize": ([_vp], _i),
     "fdtd_engine_step_range": ([_vp, _i, _i], _i),

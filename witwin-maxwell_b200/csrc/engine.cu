@@ -15,6 +15,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -79,6 +80,71 @@ int cuda_fail(cudaError_t err, const char* what) {
     cudaError_t err__ = (expr);                     \
     if (err__ != cudaSuccess) return cuda_fail(err__, #expr); \
   } while (0)
+
+// Device memory of the engines: one memory pool per device, from which an engine
+// takes its arrays in stream order.  Creating an engine makes about a hundred
+// allocations and destroying it as many frees; cudaMalloc and cudaFree take 50 us to
+// milliseconds each and wait for the device (65^3: 11 of a 20 ms solve; one
+// iteration of the 160 x 160 x 96 design with 16 checkpoints: 200 to 700 ms).
+// What a destroyed engine gave back stays in the pool up to kPoolKeep, and goes back
+// to the device beyond it at the next synchronisation.
+constexpr uint64_t kPoolKeep = 4ull << 30;
+constexpr int kMaxDevices = 64;
+
+cudaError_t device_pool(cudaMemPool_t* out) {
+  static std::mutex lock;
+  static cudaMemPool_t pools[kMaxDevices] = {};
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
+  if (dev >= kMaxDevices) return cudaErrorInvalidDevice;
+  const std::lock_guard<std::mutex> guard(lock);
+  if (!pools[dev]) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    err = cudaMemPoolCreate(&pool, &props);
+    if (err != cudaSuccess) return err;
+    uint64_t keep = kPoolKeep;
+    err = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (err != cudaSuccess) {
+      cudaMemPoolDestroy(pool);
+      return err;
+    }
+    pools[dev] = pool;
+  }
+  *out = pools[dev];
+  return cudaSuccess;
+}
+
+template <typename T>
+cudaError_t pool_alloc(T** out, size_t bytes, cudaStream_t stream) {
+  *out = nullptr;
+  cudaMemPool_t pool = nullptr;
+  cudaError_t err = device_pool(&pool);
+  if (err != cudaSuccess) return err;
+  void* p = nullptr;
+  err = cudaMallocFromPoolAsync(&p, std::max<size_t>(bytes, 1), pool, stream);
+  if (err == cudaErrorMemoryAllocation) {
+    // memory that other engines gave back on streams not yet synchronised
+    cudaGetLastError();
+    cudaDeviceSynchronize();
+    cudaMemPoolTrimTo(pool, 0);
+    err = cudaMallocFromPoolAsync(&p, std::max<size_t>(bytes, 1), pool, stream);
+  }
+  if (err == cudaSuccess) *out = static_cast<T*>(p);
+  return err;
+}
+
+void pool_free(void* p, cudaStream_t stream) {
+  if (p && cudaFreeAsync(p, stream) != cudaSuccess) {
+    cudaGetLastError();  // the caller's stream is gone: free in device order
+    cudaFree(p);
+  }
+}
 
 int axis_a(int comp) { return comp == 0 ? 1 : 0; }
 int axis_b(int comp) { return comp == 2 ? 1 : 2; }
@@ -796,7 +862,7 @@ int dev_alloc(fdtd_engine* h, float** out, size_t n) {
     *out = nullptr;
     return 0;
   }
-  CUDA_TRY(cudaMalloc(out, n * sizeof(float)));
+  CUDA_TRY(pool_alloc(out, n * sizeof(float), h->stream));
   CUDA_TRY(cudaMemsetAsync(*out, 0, n * sizeof(float), h->stream));
   h->owned.push_back(*out);
   return 0;
@@ -850,13 +916,13 @@ int background_value(fdtd_engine* h, int comp, const float* arr, float* out) {
   int ext[3];
   comp_extent(comp, h->NX, h->NY, h->NZ, ext);
   float* d = nullptr;
-  CUDA_TRY(cudaMalloc(&d, sizeof(float) * kSamples));
+  CUDA_TRY(pool_alloc(&d, sizeof(float) * kSamples, h->stream));
   coef_sample_kernel<<<kSamples / 256, 256, 0, h->stream>>>(arr, h->NY, h->P, ext[0], ext[1], ext[2], kSamples, d);
   std::vector<float> v(kSamples);
   cudaError_t err = cudaGetLastError();
   if (err == cudaSuccess) err = cudaMemcpyAsync(v.data(), d, sizeof(float) * kSamples, cudaMemcpyDeviceToHost, h->stream);
   if (err == cudaSuccess) err = cudaStreamSynchronize(h->stream);
-  cudaFree(d);
+  pool_free(d, h->stream);
   if (err != cudaSuccess) return cuda_fail(err, "coefficient background sample");
   std::sort(v.begin(), v.end());
   float best = v[0];
@@ -1452,10 +1518,10 @@ int flush_samples(fdtd_engine* h) {
 
 template <typename T>
 int upload_vec(fdtd_engine* h, T** dptr, const std::vector<T>& v) {
-  if (*dptr) cudaFree(*dptr);
+  if (*dptr) pool_free(*dptr, h->stream);
   *dptr = nullptr;
   if (v.empty()) return 0;
-  CUDA_TRY(cudaMalloc(dptr, v.size() * sizeof(T)));
+  CUDA_TRY(pool_alloc(dptr, v.size() * sizeof(T), h->stream));
   CUDA_TRY(cudaMemcpyAsync(*dptr, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, h->stream));
   return 0;
 }
@@ -1476,7 +1542,7 @@ void build_plane_csr(int NX, const std::vector<T>& items, std::vector<int>& ptr,
 int upload_ints(fdtd_engine* h, const std::vector<int>& v, const int** out) {
   int* d = nullptr;
   const size_t n = std::max<size_t>(v.size(), 1);
-  CUDA_TRY(cudaMalloc(&d, n * sizeof(int)));
+  CUDA_TRY(pool_alloc(&d, n * sizeof(int), h->stream));
   CUDA_TRY(cudaMemsetAsync(d, 0, n * sizeof(int), h->stream));
   if (!v.empty()) CUDA_TRY(cudaMemcpyAsync(d, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
   h->index_bufs.push_back(d);
@@ -1530,6 +1596,13 @@ int build_box_index(fdtd_engine* h, const std::vector<T>& items, const std::vect
 extern "C" {
 
 const char* fdtd_last_error(void) { return g_last_error.c_str(); }
+int fdtd_release_memory(uint64_t keep_bytes) {
+  cudaMemPool_t pool = nullptr;
+  CUDA_TRY(device_pool(&pool));
+  CUDA_TRY(cudaDeviceSynchronize());
+  CUDA_TRY(cudaMemPoolTrimTo(pool, static_cast<size_t>(keep_bytes)));
+  return 0;
+}
 const char* fdtd_version(void) { return "fdtd_b200 0.1.0 (sm_100a)"; }
 
 int fdtd_engine_create(const fdtd_grid_desc* desc, void* stream, fdtd_engine** out) {
@@ -1648,41 +1721,42 @@ int fdtd_engine_create(const fdtd_grid_desc* desc, void* stream, fdtd_engine** o
 int fdtd_engine_destroy(fdtd_engine* h) {
   if (!h) return 0;
   cudaStreamSynchronize(h->stream);
-  for (float* p : h->owned) cudaFree(p);
+  // work on the engine's own streams reads the arrays too
+  if (h->aux) cudaStreamSynchronize(h->aux);
+  if (h->adj.rev) cudaStreamSynchronize(h->adj.rev);
+  for (float* p : h->owned) pool_free(p, h->stream);
   for (auto& pl : h->poles) {
-    cudaFree(pl.drive);
-    cudaFree(pl.inv_eps);
-    cudaFree(pl.pol);
-    cudaFree(pl.cur);
+    pool_free(pl.drive, h->stream);
+    pool_free(pl.inv_eps, h->stream);
+    pool_free(pl.pol, h->stream);
+    pool_free(pl.cur, h->stream);
   }
   for (auto& l : h->lines) {
-    cudaFree(l.e_hist);
-    cudaFree(l.h_hist);
+    pool_free(l.e_hist, h->stream);
+    pool_free(l.h_hist, h->stream);
   }
-  for (auto& ck : h->checkpoints) cudaFree(ck.store);
-  cudaFree(h->d_terms);
-  cudaFree(h->d_poles);
-  cudaFree(h->d_regions);
-  for (int* p : h->index_bufs) cudaFree(p);
-  cudaFree(h->d_flush);
-  cudaFree(h->d_warp_class);
-  cudaFree(h->d_quad_class);
-  for (float* p : h->adj.bufs) cudaFree(p);
-  cudaFree(h->d_status);
-  cudaFree(h->d_base);
-  cudaFree(h->samples);
-  cudaFree(h->w_e);
-  cudaFree(h->w_h);
-  cudaFree(h->acc_re);
-  cudaFree(h->acc_im);
-  cudaFree(h->cmp_re);
-  cudaFree(h->cmp_im);
-  cudaFree(h->d_spectra);
-  if (h->aux) cudaStreamSynchronize(h->aux);
+  for (auto& ck : h->checkpoints) pool_free(ck.store, h->stream);
+  pool_free(h->d_terms, h->stream);
+  pool_free(h->d_poles, h->stream);
+  pool_free(h->d_regions, h->stream);
+  for (int* p : h->index_bufs) pool_free(p, h->stream);
+  pool_free(h->d_flush, h->stream);
+  pool_free(h->d_warp_class, h->stream);
+  pool_free(h->d_quad_class, h->stream);
+  for (float* p : h->adj.bufs) pool_free(p, h->stream);
+  pool_free(h->d_status, h->stream);
+  pool_free(h->d_base, h->stream);
+  pool_free(h->samples, h->stream);
+  pool_free(h->w_e, h->stream);
+  pool_free(h->w_h, h->stream);
+  pool_free(h->acc_re, h->stream);
+  pool_free(h->acc_im, h->stream);
+  pool_free(h->cmp_re, h->stream);
+  pool_free(h->cmp_im, h->stream);
+  pool_free(h->d_spectra, h->stream);
   for (cudaEvent_t e : {h->ev_fork, h->ev_join, h->ev_gat[0], h->ev_gat[1]})
     if (e) cudaEventDestroy(e);
   if (h->aux) cudaStreamDestroy(h->aux);
-  if (h->adj.rev) cudaStreamSynchronize(h->adj.rev);
   for (cudaEvent_t e : {h->adj.ev_rep[0], h->adj.ev_rep[1], h->adj.ev_rev[0], h->adj.ev_rev[1]})
     if (e) cudaEventDestroy(e);
   if (h->adj.rev) cudaStreamDestroy(h->adj.rev);
@@ -1713,7 +1787,7 @@ int fdtd_engine_set_storage(fdtd_engine* h, int kind, const float* scales) {
         for (float** buf : {&h->E[b][c], &h->H[b][c]}) {
           auto it = std::find(h->owned.begin(), h->owned.end(), *buf);
           if (it != h->owned.end()) h->owned.erase(it);
-          cudaFree(*buf);
+          pool_free(*buf, h->stream);
           *buf = nullptr;
         }
     h->storage = kind;
@@ -1895,10 +1969,10 @@ int fdtd_engine_add_pole(fdtd_engine* h, int comp, int kind, const int* box, con
   ph.state_floats =
       static_cast<int64_t>((static_cast<size_t>(rows) * nkk * (h->storage == kStoreBF16 ? 2 : 4) + 3) / 4);
   const size_t sbytes = static_cast<size_t>(ph.state_floats) * sizeof(float);
-  CUDA_TRY(cudaMalloc(&ph.drive, bytes));
-  CUDA_TRY(cudaMalloc(&ph.inv_eps, bytes));
-  CUDA_TRY(cudaMalloc(&ph.pol, sbytes));
-  CUDA_TRY(cudaMalloc(&ph.cur, sbytes));
+  CUDA_TRY(pool_alloc(&ph.drive, bytes, h->stream));
+  CUDA_TRY(pool_alloc(&ph.inv_eps, bytes, h->stream));
+  CUDA_TRY(pool_alloc(&ph.pol, sbytes, h->stream));
+  CUDA_TRY(pool_alloc(&ph.cur, sbytes, h->stream));
   CUDA_TRY(cudaMemsetAsync(ph.drive, 0, bytes, h->stream));
   CUDA_TRY(cudaMemsetAsync(ph.inv_eps, 0, bytes, h->stream));
   CUDA_TRY(cudaMemsetAsync(ph.pol, 0, sbytes, h->stream));
@@ -2109,8 +2183,8 @@ int fdtd_engine_add_aux_line(fdtd_engine* h, int n_e, const float* e_decay, cons
   AuxLine l;
   l.ne = n_e;
   l.n_steps = n_steps;
-  CUDA_TRY(cudaMalloc(&l.e_hist, sizeof(float) * static_cast<size_t>(n_steps) * n_e));
-  CUDA_TRY(cudaMalloc(&l.h_hist, sizeof(float) * static_cast<size_t>(n_steps) * n_e));
+  CUDA_TRY(pool_alloc(&l.e_hist, sizeof(float) * static_cast<size_t>(n_steps) * n_e, h->stream));
+  CUDA_TRY(pool_alloc(&l.h_hist, sizeof(float) * static_cast<size_t>(n_steps) * n_e, h->stream));
   float *ed, *ecu, *hd, *hcu, *src, *e, *hh;
   int rc = dev_copy(h, &ed, e_decay, n_e);
   if (!rc) rc = dev_copy(h, &ecu, e_curl, n_e);
@@ -2152,12 +2226,13 @@ int fdtd_engine_add_line_patch(fdtd_engine* h, int comp, const int* box, const f
   // Every sample index must address a stored entry of the line history: E
   // histories hold n_e values per step, H histories n_e - 1.
   std::vector<int> host_idx(axis_len);
+  CUDA_TRY(cudaStreamSynchronize(h->stream));
   CUDA_TRY(cudaMemcpy(host_idx.data(), sample_index, sizeof(int) * axis_len, cudaMemcpyDefault));
   const int limit = sample_kind == 0 ? l.ne : l.ne - 1;
   for (int v : host_idx)
     if (v < 0 || v >= limit) return fail(FDTD_ERR_INVALID_ARG, "line patch sample index outside the incident line");
   int* idx = nullptr;
-  CUDA_TRY(cudaMalloc(&idx, sizeof(int) * axis_len));
+  CUDA_TRY(pool_alloc(&idx, sizeof(int) * axis_len, h->stream));
   CUDA_TRY(cudaMemcpyAsync(idx, host_idx.data(), sizeof(int) * axis_len, cudaMemcpyHostToDevice, h->stream));
   CUDA_TRY(cudaStreamSynchronize(h->stream));
   h->owned.push_back(reinterpret_cast<float*>(idx));
@@ -2200,22 +2275,22 @@ int set_dft_impl(fdtd_engine* h, int n_freq, const double* omega, int n_steps, c
     return fail(FDTD_ERR_INVALID_ARG, "bad DFT arguments");
   h->n_freq = n_freq;
   h->dft_steps = n_steps;
-  cudaFree(h->w_e);
-  cudaFree(h->w_h);
-  CUDA_TRY(cudaMalloc(&h->w_e, sizeof(float2) * static_cast<size_t>(n_freq) * n_steps));
-  CUDA_TRY(cudaMalloc(&h->w_h, sizeof(float2) * static_cast<size_t>(n_freq) * n_steps));
+  pool_free(h->w_e, h->stream);
+  pool_free(h->w_h, h->stream);
+  CUDA_TRY(pool_alloc(&h->w_e, sizeof(float2) * static_cast<size_t>(n_freq) * n_steps, h->stream));
+  CUDA_TRY(pool_alloc(&h->w_h, sizeof(float2) * static_cast<size_t>(n_freq) * n_steps, h->stream));
   const size_t n_window = static_cast<size_t>(n_steps) * (per_freq ? n_freq : 1);
   double *d_omega = nullptr, *d_window = nullptr;
-  CUDA_TRY(cudaMalloc(&d_omega, sizeof(double) * n_freq));
-  CUDA_TRY(cudaMalloc(&d_window, sizeof(double) * n_window));
+  CUDA_TRY(pool_alloc(&d_omega, sizeof(double) * n_freq, h->stream));
+  CUDA_TRY(pool_alloc(&d_window, sizeof(double) * n_window, h->stream));
   CUDA_TRY(cudaMemcpyAsync(d_omega, omega, sizeof(double) * n_freq, cudaMemcpyHostToDevice, h->stream));
   CUDA_TRY(cudaMemcpyAsync(d_window, window, sizeof(double) * n_window, cudaMemcpyHostToDevice, h->stream));
   dft_weight_kernel<<<256, 256, 0, h->stream>>>(n_freq, n_steps, d_omega, d_window, per_freq, h->desc.dt, h->w_e,
                                                 h->w_h);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaStreamSynchronize(h->stream));
-  cudaFree(d_omega);
-  cudaFree(d_window);
+  pool_free(d_omega, h->stream);
+  pool_free(d_window, h->stream);
   return 0;
 }
 
@@ -2287,6 +2362,7 @@ int estimate_scales(fdtd_engine* h) {
 int fdtd_engine_finalize(fdtd_engine* h) {
   if (!h) return fail(FDTD_ERR_INVALID_ARG, "null engine");
   if (h->finalized) return 0;
+  CUDA_TRY(cudaStreamSynchronize(h->stream));  // the synchronous reads below follow the uploads
   if (h->storage == kStoreF16 && !h->scales_set) {
     const int rc = estimate_scales(h);
     if (rc) return rc;
@@ -2337,8 +2413,9 @@ int fdtd_engine_finalize(fdtd_engine* h) {
         return fail(FDTD_ERR_UNSUPPORTED, "nonlinear media with poles run launch variants 1-3, 10 and 11");
     }
     const int64_t n = static_cast<int64_t>(h->nl_cells_h.size() / 4);
-    CUDA_TRY(cudaMalloc(&h->d_nl_cells, sizeof(int4) * n));
+    CUDA_TRY(pool_alloc(&h->d_nl_cells, sizeof(int4) * n, h->stream));
     h->owned.push_back(reinterpret_cast<float*>(h->d_nl_cells));
+    CUDA_TRY(cudaStreamSynchronize(h->stream));
     CUDA_TRY(cudaMemcpy(h->d_nl_cells, h->nl_cells_h.data(), sizeof(int4) * n, cudaMemcpyHostToDevice));
     std::vector<float> prm;
     prm.reserve(static_cast<size_t>(6 * n));
@@ -2480,6 +2557,7 @@ int fdtd_engine_finalize(fdtd_engine* h) {
       for (int i = 0; i < h->NX; ++i)
         if (ptr_host[i + 1] > ptr_host[i]) bits[i] |= static_cast<int>(flag);
     };
+    CUDA_TRY(cudaStreamSynchronize(h->stream));
     for (int ph = 0; ph < 2; ++ph) {
       std::vector<int> pt(h->NX + 1), pr(h->NX + 1);
       CUDA_TRY(cudaMemcpy(pt.data(), h->term_ix[ph].ptr[0], sizeof(int) * (h->NX + 1), cudaMemcpyDeviceToHost));
@@ -2511,13 +2589,13 @@ int fdtd_engine_finalize(fdtd_engine* h) {
   if (rc) return rc;
   h->n_flush = static_cast<int>(fl.size());
   if (h->n_samples > 0) {
-    CUDA_TRY(cudaMalloc(&h->samples, sizeof(float) * static_cast<size_t>(h->M) * h->n_samples));
+    CUDA_TRY(pool_alloc(&h->samples, sizeof(float) * static_cast<size_t>(h->M) * h->n_samples, h->stream));
     if (h->n_freq > 0) {
       const size_t acc = static_cast<size_t>(h->n_freq) * h->n_samples;
-      CUDA_TRY(cudaMalloc(&h->acc_re, sizeof(float) * acc));
-      CUDA_TRY(cudaMalloc(&h->acc_im, sizeof(float) * acc));
-      CUDA_TRY(cudaMalloc(&h->cmp_re, sizeof(float) * acc));
-      CUDA_TRY(cudaMalloc(&h->cmp_im, sizeof(float) * acc));
+      CUDA_TRY(pool_alloc(&h->acc_re, sizeof(float) * acc, h->stream));
+      CUDA_TRY(pool_alloc(&h->acc_im, sizeof(float) * acc, h->stream));
+      CUDA_TRY(pool_alloc(&h->cmp_re, sizeof(float) * acc, h->stream));
+      CUDA_TRY(pool_alloc(&h->cmp_im, sizeof(float) * acc, h->stream));
       CUDA_TRY(cudaMemsetAsync(h->acc_re, 0, sizeof(float) * acc, h->stream));
       CUDA_TRY(cudaMemsetAsync(h->acc_im, 0, sizeof(float) * acc, h->stream));
       CUDA_TRY(cudaMemsetAsync(h->cmp_re, 0, sizeof(float) * acc, h->stream));
@@ -2539,11 +2617,11 @@ int fdtd_engine_finalize(fdtd_engine* h) {
   }
   {
     const int64_t kblocks = (h->NZ + kWarpOut - 1) / kWarpOut;
-    CUDA_TRY(cudaMalloc(&h->d_warp_class, static_cast<size_t>(h->NX) * kblocks * h->NY));
+    CUDA_TRY(pool_alloc(&h->d_warp_class, static_cast<size_t>(h->NX) * kblocks * h->NY, h->stream));
     h->class_key = 0;
     h->quad_key = 0;
     if (h->storage == kStoreF32 && has_coef(h))
-      CUDA_TRY(cudaMalloc(&h->d_quad_class, static_cast<size_t>(h->NX) * h->NY * (h->P / 4)));
+      CUDA_TRY(pool_alloc(&h->d_quad_class, static_cast<size_t>(h->NX) * h->NY * (h->P / 4), h->stream));
     if (h->storage == kStoreF32) {
       rc = dev_alloc(h, &h->d_ztab_h, 4 * static_cast<size_t>(h->P));
       if (!rc) rc = dev_alloc(h, &h->d_ztab_e, 4 * static_cast<size_t>(h->P));
@@ -2555,9 +2633,9 @@ int fdtd_engine_finalize(fdtd_engine* h) {
         err = launch_quad_ztable(h->eb[2], h->ec[2], h->eik[2], h->inv_e[2], h->NZ, lo, hi, h->P, h->d_ztab_e, h->stream);
       if (err != 0) return cuda_fail(static_cast<cudaError_t>(err), "quad_ztable_kernel launch");
     }
-    CUDA_TRY(cudaMalloc(&h->d_status, sizeof(int)));
+    CUDA_TRY(pool_alloc(&h->d_status, sizeof(int), h->stream));
     CUDA_TRY(cudaMemsetAsync(h->d_status, 0, sizeof(int), h->stream));
-    CUDA_TRY(cudaMalloc(&h->d_base, sizeof(int)));
+    CUDA_TRY(pool_alloc(&h->d_base, sizeof(int), h->stream));
     CUDA_TRY(cudaMemsetAsync(h->d_base, 0, sizeof(int), h->stream));
   }
   {
@@ -2767,13 +2845,13 @@ static void state_buffers(fdtd_engine* h, std::vector<std::pair<float*, size_t>>
   }
 }
 
-static int checkpoint_alloc(Checkpoint& ck, const std::vector<std::pair<float*, size_t>>& bufs) {
+static int checkpoint_alloc(fdtd_engine* h, Checkpoint& ck, const std::vector<std::pair<float*, size_t>>& bufs) {
   if (ck.store && ck.bufs.size() == bufs.size()) return 0;
-  cudaFree(ck.store);
+  pool_free(ck.store, h->stream);
   ck.store = nullptr;
   size_t total = 0;
   for (const auto& b : bufs) total += (b.second + 63) / 64 * 64;  // 256-byte aligned views
-  CUDA_TRY(cudaMalloc(&ck.store, std::max<size_t>(total, 1) * sizeof(float)));
+  CUDA_TRY(pool_alloc(&ck.store, std::max<size_t>(total, 1) * sizeof(float), h->stream));
   ck.bufs.clear();
   size_t off = 0;
   for (const auto& b : bufs) {
@@ -2789,7 +2867,7 @@ int fdtd_engine_checkpoint_reserve(fdtd_engine* h, int n_slots) {
   std::vector<std::pair<float*, size_t>> bufs;
   state_buffers(h, bufs);
   for (int s = 0; s < n_slots; ++s) {
-    int rc = checkpoint_alloc(h->checkpoints[s], bufs);
+    int rc = checkpoint_alloc(h, h->checkpoints[s], bufs);
     if (rc) return rc;
   }
   return 0;
@@ -2802,7 +2880,7 @@ int fdtd_engine_checkpoint_save(fdtd_engine* h, int slot) {
   std::vector<std::pair<float*, size_t>> bufs;
   state_buffers(h, bufs);
   Checkpoint& ck = h->checkpoints[slot];
-  int rc = checkpoint_alloc(ck, bufs);
+  int rc = checkpoint_alloc(h, ck, bufs);
   if (rc) return rc;
   for (size_t x = 0; x < bufs.size(); ++x)
     CUDA_TRY(cudaMemcpyAsync(ck.bufs[x], bufs[x].first, bufs[x].second * sizeof(float), cudaMemcpyDeviceToDevice,
@@ -2881,7 +2959,7 @@ int fdtd_engine_autotune(fdtd_engine* h, int* tile_rows, int* chunk_planes) {
   h->TY = best_ty;
   rc = fdtd_engine_checkpoint_load(h, slot);
   if (rc) return rc;
-  cudaFree(h->checkpoints[slot].store);
+  pool_free(h->checkpoints[slot].store, h->stream);
   h->checkpoints.pop_back();
   h->pending = 0;
   h->pending_base = next_step;
@@ -3014,7 +3092,7 @@ int fdtd_engine_set_prefetch(fdtd_engine* h, int planes) {
 static int adj_alloc(fdtd_engine* h, float** out, size_t n) {
   *out = nullptr;
   if (n == 0) return 0;
-  CUDA_TRY(cudaMalloc(out, n * sizeof(float)));
+  CUDA_TRY(pool_alloc(out, n * sizeof(float), h->stream));
   CUDA_TRY(cudaMemsetAsync(*out, 0, n * sizeof(float), h->stream));
   h->adj.bufs.push_back(*out);
   return 0;
@@ -3053,10 +3131,11 @@ int fdtd_engine_adjoint_init(fdtd_engine* h, const int* design_boxes, int max_se
     }
     float** dgp = nullptr;
     float** dgc = nullptr;
-    CUDA_TRY(cudaMalloc(&dgp, sizeof(float*) * gp.size()));
+    CUDA_TRY(pool_alloc(&dgp, sizeof(float*) * gp.size(), h->stream));
     a.bufs.push_back(reinterpret_cast<float*>(dgp));
-    CUDA_TRY(cudaMalloc(&dgc, sizeof(float*) * gc.size()));
+    CUDA_TRY(pool_alloc(&dgc, sizeof(float*) * gc.size(), h->stream));
     a.bufs.push_back(reinterpret_cast<float*>(dgc));
+    CUDA_TRY(cudaStreamSynchronize(h->stream));
     CUDA_TRY(cudaMemcpy(dgp, gp.data(), sizeof(float*) * gp.size(), cudaMemcpyHostToDevice));
     CUDA_TRY(cudaMemcpy(dgc, gc.data(), sizeof(float*) * gc.size(), cudaMemcpyHostToDevice));
     a.q.gpol = dgp;
@@ -3537,11 +3616,12 @@ int fdtd_batch_create(fdtd_engine* const* engines, int n, void* stream, fdtd_bat
     err = cudaStreamCreateWithFlags(&b->streams[i], cudaStreamNonBlocking);
     if (err == cudaSuccess) err = cudaEventCreateWithFlags(&b->join[i], cudaEventDisableTiming);
   }
-  if (err == cudaSuccess) err = cudaMalloc(&b->d_bases, sizeof(int*) * n);
+  if (err == cudaSuccess) err = pool_alloc(&b->d_bases, sizeof(int*) * n, b->stream);
   if (err == cudaSuccess) {
     std::vector<int*> bases(n);
     for (int i = 0; i < n; ++i) bases[i] = engines[i]->d_base;
-    err = cudaMemcpy(b->d_bases, bases.data(), sizeof(int*) * n, cudaMemcpyHostToDevice);
+    err = cudaStreamSynchronize(b->stream);
+    if (err == cudaSuccess) err = cudaMemcpy(b->d_bases, bases.data(), sizeof(int*) * n, cudaMemcpyHostToDevice);
   }
   if (err != cudaSuccess) {
     const int rc = cuda_fail(err, "batch create");
@@ -3564,7 +3644,7 @@ int fdtd_batch_destroy(fdtd_batch* b) {
   if (b->fork) cudaEventDestroy(b->fork);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
-  cudaFree(b->d_bases);
+  pool_free(b->d_bases, b->stream);
   delete b;
   return 0;
 }

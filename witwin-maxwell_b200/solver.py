@@ -52,6 +52,13 @@ def pin_scene(cs):
     )
 
 
+def release_memory(keep_bytes: int = 0, device=None) -> None:
+    """Give the device memory that closed solvers left in the library's pool (at most
+    4 GiB) back to the device, but for ``keep_bytes``."""
+    with torch.cuda.device(torch.device("cuda") if device is None else torch.device(device)):
+        _lib.check(_lib.load().fdtd_release_memory(int(keep_bytes)), "release_memory")
+
+
 class B200FDTD:
     def __init__(
         self,
