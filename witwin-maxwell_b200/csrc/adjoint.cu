@@ -23,6 +23,9 @@
 //   dE'/deps = -(ce curl + S - A) / eps = -(E^{n+1} - de E^n) ce / dt,
 // evaluated from the replayed E history of the box.  Sources are affine in the
 // fields: they add nothing to the adjoint recursion itself.
+#include <algorithm>
+#include <climits>
+
 #include <cuda_runtime.h>
 
 #include "../../include/fdtd_b200.h"
@@ -132,12 +135,8 @@ __device__ __forceinline__ bool plain_cell(const StepParams& p, int i, int j, in
 
 // ---- pass A: gH_mid = gH + C_H^T g(d_E) (in place in q.gH) ----
 template <bool kUniform>
-__global__ void adj_pass_a_kernel(const StepParams p, const AdjParams q) {
+__device__ __forceinline__ void pass_a_cell(const StepParams& p, const AdjParams& q, int i, int j, int k) {
   {
-    // one thread per cell: k from the x-dimension, rows and planes from y and z
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, i = blockIdx.z;
-    if (k >= p.P) return;
     const int64_t x = (static_cast<int64_t>(i) * p.NY + j) * p.P + k;
     const float* iex = p.inv_e[0];
     const float* iey = p.inv_e[1];
@@ -207,12 +206,8 @@ __global__ void adj_pass_a_kernel(const StepParams p, const AdjParams q) {
 // 782 ms.  The pole kernel spills at that budget and runs five CTAs per SM
 // (at most 102 registers, 70-72 used).
 template <bool kUniform, bool kPoles>
-__global__ void __launch_bounds__(128, kPoles ? 5 : 12) adj_pass_b_kernel(const StepParams p, const AdjParams q) {
+__device__ __forceinline__ void pass_b_cell(const StepParams& p, const AdjParams& q, int i, int j, int k) {
   {
-    // one thread per cell: k from the x-dimension, rows and planes from y and z
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, i = blockIdx.z;
-    if (k >= p.P) return;
     const int64_t x = (static_cast<int64_t>(i) * p.NY + j) * p.P + k;
     const float* ihx = p.inv_h[0];
     const float* ihy = p.inv_h[1];
@@ -341,12 +336,8 @@ __global__ void __launch_bounds__(128, kPoles ? 5 : 12) adj_pass_b_kernel(const 
 }
 
 // ---- pass C: adjoint H psi; gH = dh gH_mid ----
-__global__ void adj_pass_c_kernel(const StepParams p, const AdjParams q) {
+__device__ __forceinline__ void pass_c_cell(const StepParams& p, const AdjParams& q, int i, int j, int k) {
   {
-    // one thread per cell: k from the x-dimension, rows and planes from y and z
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, i = blockIdx.z;
-    if (k >= p.P) return;
     const int64_t x = (static_cast<int64_t>(i) * p.NY + j) * p.P + k;
     // cells outside every slab have nothing to do when no H component decays
     bool unit = true;
@@ -384,6 +375,237 @@ __global__ void adj_pass_c_kernel(const StepParams p, const AdjParams q) {
       q.gH[c][x] = coef(p.hdecay[c], p.hdecay_u[c], x) * gm;
     }
   }
+}
+
+// The cells of the padded grid outside the box [x0, x1) x [y0, y1) x [k0, k1), in
+// six blocks; end[b]: cells of blocks 0 .. b.
+struct Shell {
+  int x0, x1, y0, y1, k0, k1;
+  int end[6];
+};
+__device__ __forceinline__ bool shell_cell(const StepParams& p, const Shell& s, int t, int& i, int& j, int& k) {
+  if (t >= s.end[5]) return false;
+  int b = 0;
+  while (t >= s.end[b]) ++b;
+  if (b) t -= s.end[b - 1];
+  const int i_lo = b == 0 ? 0 : (b == 1 ? s.x1 : s.x0);
+  const int j_lo = b < 2 || b == 2 ? 0 : (b == 3 ? s.y1 : s.y0);
+  const int k_lo = b == 5 ? s.k1 : 0;
+  const int nj = b < 2 ? p.NY : (b == 2 ? s.y0 : (b == 3 ? p.NY - s.y1 : s.y1 - s.y0));
+  const int nk = b < 4 ? p.P : (b == 4 ? s.k0 : p.P - s.k1);
+  const int r = t / nk;
+  k = k_lo + t - r * nk;
+  i = i_lo + r / nj;
+  j = j_lo + r - r / nj * nj;
+  return true;
+}
+
+// Passes A and B on the cells of the box [x0, x1) x [y0, y1) x [k0, k1) (k0, k1
+// multiples of four), every one a plain cell: a thread takes four consecutive z
+// cells, so that a neighbour read is one 16-byte load for the four (and one value
+// for the shifted cell).  Both passes are bound by instruction issue and L2 latency:
+// one cell per thread took 97 and 137 us per step of the 160 x 160 x 96 design, whose
+// state stays in L2.  The cells around the box (slabs, faces) stay one per thread.
+struct Box {
+  int x0, x1, y0, y1, k0, k1;
+};
+__device__ __forceinline__ bool box_quad(const StepParams& p, const Box& b, int& i, int& j, int& k, int64_t& x) {
+  const int nq = (b.k1 - b.k0) >> 2, ny = b.y1 - b.y0;
+  const int t = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+  const int r = t / nq;
+  i = b.x0 + r / ny;
+  if (i >= b.x1) return false;
+  j = b.y0 + r - r / ny * ny;
+  k = b.k0 + 4 * (t - r * nq);
+  x = cell(p, i, j, k);
+  return true;
+}
+__device__ __forceinline__ void load4(float (&v)[4], const float* a) {
+  const float4 f = *reinterpret_cast<const float4*>(a);
+  v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+}
+__device__ __forceinline__ void store4(float* a, const float (&v)[4]) {
+  *reinterpret_cast<float4*>(a) = make_float4(v[0], v[1], v[2], v[3]);
+}
+// coefficient times adjoint field of the four cells at x
+__device__ __forceinline__ void scaled4(float (&v)[4], const float* arr, float uni, const float* g, int64_t x) {
+  load4(v, g + x);
+  if (arr) {
+    float c[4];
+    load4(c, arr + x);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) v[a] = c[a] * v[a];
+  } else {
+#pragma unroll
+    for (int a = 0; a < 4; ++a) v[a] = uni * v[a];
+  }
+}
+
+template <bool kUniform>
+__device__ __forceinline__ void box_a(const StepParams& p, const AdjParams& q, const Box& box) {
+  int i, j, k;
+  int64_t x;
+  if (!box_quad(p, box, i, j, k, x)) return;
+  const int64_t sy = p.P, sx = static_cast<int64_t>(p.NY) * p.P;
+  float ux[5], uy[5], uz[4], uxj[4], uyi[4], uzj[4], uzi[4], t[4];
+  scaled4(t, p.ecurl[0], p.ecurl_u[0], q.gE[0], x);
+#pragma unroll
+  for (int a = 0; a < 4; ++a) ux[a] = t[a];
+  ux[4] = coef(p.ecurl[0], p.ecurl_u[0], x + 4) * q.gE[0][x + 4];
+  scaled4(t, p.ecurl[1], p.ecurl_u[1], q.gE[1], x);
+#pragma unroll
+  for (int a = 0; a < 4; ++a) uy[a] = t[a];
+  uy[4] = coef(p.ecurl[1], p.ecurl_u[1], x + 4) * q.gE[1][x + 4];
+  scaled4(uz, p.ecurl[2], p.ecurl_u[2], q.gE[2], x);
+  scaled4(uxj, p.ecurl[0], p.ecurl_u[0], q.gE[0], x + sy);
+  scaled4(uyi, p.ecurl[1], p.ecurl_u[1], q.gE[1], x + sx);
+  scaled4(uzj, p.ecurl[2], p.ecurl_u[2], q.gE[2], x + sy);
+  scaled4(uzi, p.ecurl[2], p.ecurl_u[2], q.gE[2], x + sx);
+  const float ey0 = inv_at<kUniform>(p.inv_e[1], j, p.NY, p.inv_e_u[1]);
+  const float ey1 = inv_at<kUniform>(p.inv_e[1], j + 1, p.NY, p.inv_e_u[1]);
+  const float ex0 = inv_at<kUniform>(p.inv_e[0], i, p.NX, p.inv_e_u[0]);
+  const float ex1 = inv_at<kUniform>(p.inv_e[0], i + 1, p.NX, p.inv_e_u[0]);
+  float hx[4], hy[4], hz[4];
+  load4(hx, q.gH[0] + x);
+  load4(hy, q.gH[1] + x);
+  load4(hz, q.gH[2] + x);
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const float ez0 = inv_at<kUniform>(p.inv_e[2], k + a, p.NZ, p.inv_e_u[2]);
+    const float ez1 = inv_at<kUniform>(p.inv_e[2], k + a + 1, p.NZ, p.inv_e_u[2]);
+    hx[a] += ez0 * uy[a] - ez1 * uy[a + 1];
+    hx[a] += ey0 * -uz[a] - ey1 * -uzj[a];
+    hy[a] += ez0 * -ux[a] - ez1 * -ux[a + 1];
+    hy[a] += ex0 * uz[a] - ex1 * uzi[a];
+    hz[a] += ey0 * ux[a] - ey1 * uxj[a];
+    hz[a] += ex0 * -uy[a] - ex1 * -uyi[a];
+  }
+  store4(q.gH[0] + x, hx);
+  store4(q.gH[1] + x, hy);
+  store4(q.gH[2] + x, hz);
+}
+
+// dL/deps of the cells of a quad that lie in component c's design box (see pass B).
+__device__ __forceinline__ void design_quad(const StepParams& p, const AdjParams& q, int c, int i, int j, int k,
+                                            int64_t x, const float (&gp)[4]) {
+  const DesignBox& d = q.design[c];
+  if (!d.grad || i < d.lo[0] || i >= d.hi[0] || j < d.lo[1] || j >= d.hi[1] || k + 4 <= d.lo[2] || k >= d.hi[2]) return;
+  const int64_t row = (static_cast<int64_t>(i - d.lo[0]) * (d.hi[1] - d.lo[1]) + (j - d.lo[1])) * (d.hi[2] - d.lo[2]);
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    if (k + a < d.lo[2] || k + a >= d.hi[2]) continue;
+    const int64_t l = row + (k + a - d.lo[2]);
+    const float e_next = d.hist[static_cast<int64_t>(q.hist_slot + 1) * d.cells + l];
+    const float e_now = d.hist[static_cast<int64_t>(q.hist_slot) * d.cells + l];
+    const float de = coef(p.edecay[c], p.edecay_u[c], x + a), ce = coef(p.ecurl[c], p.ecurl_u[c], x + a);
+    d.grad[l] += -gp[a] * (e_next - de * e_now) * ce * q.inv_dt;
+  }
+}
+
+template <bool kUniform>
+__device__ __forceinline__ void box_b(const StepParams& p, const AdjParams& q, const Box& box) {
+  int i, j, k;
+  int64_t x;
+  if (!box_quad(p, box, i, j, k, x)) return;
+  const int64_t sy = p.P, sx = static_cast<int64_t>(p.NY) * p.P;
+  float vx[4], vy[4], vz[4], w[4], gp[4], g[4], de[4], zx[5], zy[5];
+  scaled4(vx, p.hcurl[0], p.hcurl_u[0], q.gH[0], x);
+  scaled4(vy, p.hcurl[1], p.hcurl_u[1], q.gH[1], x);
+  scaled4(vz, p.hcurl[2], p.hcurl_u[2], q.gH[2], x);
+  zx[0] = coef(p.hcurl[0], p.hcurl_u[0], x - 1) * q.gH[0][x - 1];  // the cells at k - 1 + a
+  zy[0] = coef(p.hcurl[1], p.hcurl_u[1], x - 1) * q.gH[1][x - 1];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    zx[a + 1] = vx[a];
+    zy[a + 1] = vy[a];
+  }
+  const float hy0 = inv_at<kUniform>(p.inv_h[1], j, p.NY - 1, p.inv_h_u[1]);
+  const float hy1 = inv_at<kUniform>(p.inv_h[1], j - 1, p.NY - 1, p.inv_h_u[1]);
+  const float hx0 = inv_at<kUniform>(p.inv_h[0], i, p.NX - 1, p.inv_h_u[0]);
+  const float hx1 = inv_at<kUniform>(p.inv_h[0], i - 1, p.NX - 1, p.inv_h_u[0]);
+  float hz0[4], hz1[4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    hz0[a] = inv_at<kUniform>(p.inv_h[2], k + a, p.NZ - 1, p.inv_h_u[2]);
+    hz1[a] = inv_at<kUniform>(p.inv_h[2], k + a - 1, p.NZ - 1, p.inv_h_u[2]);
+  }
+#define FDTD_ADJ_DECAY(C)                                                                       \
+  do {                                                                                          \
+    load4(gp, q.gE[C] + x);                                                                     \
+    if (p.edecay[C]) load4(de, p.edecay[C] + x);                                                \
+    else de[0] = de[1] = de[2] = de[3] = p.edecay_u[C];                                         \
+    _Pragma("unroll") for (int a = 0; a < 4; ++a) g[a] = de[a] * gp[a];                         \
+  } while (0)
+  FDTD_ADJ_DECAY(0);  // Ex: Hy (z), Hz (y)
+  scaled4(w, p.hcurl[2], p.hcurl_u[2], q.gH[2], x - sy);
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    g[a] += -hz0[a] * -vy[a] + hz1[a] * -zy[a];
+    g[a] += -hy0 * vz[a] + hy1 * w[a];
+  }
+  design_quad(p, q, 0, i, j, k, x, gp);
+  store4(q.gE[0] + x, g);
+  FDTD_ADJ_DECAY(1);  // Ey: Hx (z), Hz (x)
+  scaled4(w, p.hcurl[2], p.hcurl_u[2], q.gH[2], x - sx);
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    g[a] += -hz0[a] * vx[a] + hz1[a] * zx[a];
+    g[a] += -hx0 * -vz[a] + hx1 * -w[a];
+  }
+  design_quad(p, q, 1, i, j, k, x, gp);
+  store4(q.gE[1] + x, g);
+  FDTD_ADJ_DECAY(2);  // Ez: Hx (y), Hy (x)
+  scaled4(w, p.hcurl[0], p.hcurl_u[0], q.gH[0], x - sy);
+  float u[4];
+  scaled4(u, p.hcurl[1], p.hcurl_u[1], q.gH[1], x - sx);
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    g[a] += -hy0 * -vx[a] + hy1 * -w[a];
+    g[a] += -hx0 * vy[a] + hx1 * u[a];
+  }
+  design_quad(p, q, 2, i, j, k, x, gp);
+  store4(q.gE[2] + x, g);
+#undef FDTD_ADJ_DECAY
+}
+
+// One thread per cell: of the whole grid (k from the x-dimension, rows and planes
+// from y and z; an empty shell), or of the shell after `first` blocks on the box.
+// Box and shell share a launch: one after the other they left SMs idle twice (80 x
+// 80 x 48: 59.3 against 57.8 ms for a whole gradient).
+__device__ __forceinline__ bool grid_cell(const StepParams& p, const Shell& s, int first, int& i, int& j, int& k) {
+  if (s.end[5] > 0)
+    return shell_cell(p, s, static_cast<int>((blockIdx.x - first) * blockDim.x + threadIdx.x), i, j, k);
+  k = blockIdx.x * blockDim.x + threadIdx.x;
+  j = blockIdx.y;
+  i = blockIdx.z;
+  return k < p.P;
+}
+template <bool kUniform>
+__global__ void __launch_bounds__(128)
+    adj_pass_a_kernel(const StepParams p, const AdjParams q, const Box box, const Shell s, int first) {
+  if (static_cast<int>(blockIdx.x) < first) {
+    box_a<kUniform>(p, q, box);
+    return;
+  }
+  int i, j, k;
+  if (grid_cell(p, s, first, i, j, k)) pass_a_cell<kUniform>(p, q, i, j, k);
+}
+// kPoles: the scene has ADE poles, whose transpose is written per cell only (no box).
+// The pole-free kernel runs nine 128-thread CTAs per SM (56 registers, the box body's);
+// the pole kernel five.
+template <bool kUniform, bool kPoles>
+__global__ void __launch_bounds__(128, kPoles ? 5 : 9)
+    adj_pass_b_kernel(const StepParams p, const AdjParams q, const Box box, const Shell s, int first) {
+  if (!kPoles && static_cast<int>(blockIdx.x) < first) {
+    box_b<kUniform>(p, q, box);
+    return;
+  }
+  int i, j, k;
+  if (grid_cell(p, s, first, i, j, k)) pass_b_cell<kUniform, kPoles>(p, q, i, j, k);
+}
+__global__ void adj_pass_c_kernel(const StepParams p, const AdjParams q, const Shell s) {
+  int i, j, k;
+  if (grid_cell(p, s, 0, i, j, k)) pass_c_cell(p, q, i, j, k);
 }
 
 // Monitor seeds of step n: the adjoint of the sampled value of every slot,
@@ -441,24 +663,70 @@ unsigned grid_for(int64_t n) {
 
 }  // namespace
 
+namespace {
+
+// The plain cells of a pass (plain_cell with the same floor, a0, a1), whole quads in
+// z; empty boxes have x1 <= x0.
+Box plain_box(const StepParams& p, int floor_, int a0, int a1) {
+  const int n[3] = {p.NX, p.NY, p.NZ};
+  int lo[3], hi[3];
+  for (int a = 0; a < 3; ++a) {
+    lo[a] = std::max(p.cpml ? p.slab_lo[a] : 0, floor_) + a0;
+    hi[a] = n[a] - std::max(p.cpml ? p.slab_hi[a] : 0, floor_) - a1 + 1;
+  }
+  Box b{lo[0], hi[0], lo[1], hi[1], (lo[2] + 3) / 4 * 4, hi[2] / 4 * 4};
+  const int64_t quads = static_cast<int64_t>(b.x1 - b.x0) * (b.y1 - b.y0) * ((b.k1 - b.k0) / 4);
+  if (b.x1 <= b.x0 || b.y1 <= b.y0 || b.k1 <= b.k0 || quads > INT_MAX) b.x1 = b.x0 = 0;
+  return b;
+}
+
+// The cells outside a box; end[5] = 0 (the whole grid) for an empty box or a grid
+// beyond 32-bit counts.
+Shell shell_of(const StepParams& p, const Box& b) {
+  Shell s{b.x0, b.x1, b.y0, b.y1, b.k0, b.k1, {0, 0, 0, 0, 0, 0}};
+  if (b.x1 <= b.x0 || static_cast<int64_t>(p.NX) * p.NY * p.P > INT_MAX) return s;
+  const int nx = b.x1 - b.x0, ny = b.y1 - b.y0, plane = p.NY * p.P;
+  const int cells[6] = {b.x0 * plane, (p.NX - b.x1) * plane, nx * b.y0 * p.P, nx * (p.NY - b.y1) * p.P,
+                        nx * ny * b.k0, nx * ny * (p.P - b.k1)};
+  int sum = 0;
+  for (int r = 0; r < 6; ++r) s.end[r] = sum += cells[r];
+  return s;
+}
+
+}  // namespace
+
 int launch_adjoint_step(const StepParams& p, const AdjParams& q, const RegionFlush* regions, int n_regions,
                         const float2* w_e, const float2* w_h, int n_freq, int n, cudaStream_t stream) {
   if (n_regions > 0 && q.seed_re) {
     dim3 grid(64, n_regions);
     adj_seed_kernel<<<grid, 256, 0, stream>>>(p, q, regions, n_regions, w_e, w_h, n_freq, n);
   }
-  const dim3 cells((p.P + 127) / 128, p.NY, p.NX);
-  const bool poles = p.n_poles > 0;
-  if (p.uniform_grid) {
-    adj_pass_a_kernel<true><<<cells, 128, 0, stream>>>(p, q);
-    if (poles) adj_pass_b_kernel<true, true><<<cells, 128, 0, stream>>>(p, q);
-    else adj_pass_b_kernel<true, false><<<cells, 128, 0, stream>>>(p, q);
+  const dim3 all((p.P + 127) / 128, p.NY, p.NX);
+  const bool poles = p.n_poles > 0, uni = p.uniform_grid != 0;
+  const Shell whole{0, 0, 0, 0, 0, 0, {0, 0, 0, 0, 0, 0}};
+  const Box none{0, 0, 0, 0, 0, 0};
+  auto quad_blocks = [](const Box& b, const Shell& s) {
+    return s.end[5] > 0 ? ((b.x1 - b.x0) * (b.y1 - b.y0) * ((b.k1 - b.k0) / 4) + 127) / 128 : 0;
+  };
+  auto blocks = [&](const Shell& s, int first) { return s.end[5] > 0 ? dim3(first + (s.end[5] + 127) / 128) : all; };
+  const Box box_a = plain_box(p, 1, 0, 2), box_b = plain_box(p, 0, 1, 2);
+  const Shell shell_a = shell_of(p, box_a), shell_b = shell_of(p, box_b);
+  const int first_a = quad_blocks(box_a, shell_a), first_b = quad_blocks(box_b, shell_b);
+  if (uni) adj_pass_a_kernel<true><<<blocks(shell_a, first_a), 128, 0, stream>>>(p, q, box_a, shell_a, first_a);
+  else adj_pass_a_kernel<false><<<blocks(shell_a, first_a), 128, 0, stream>>>(p, q, box_a, shell_a, first_a);
+  if (poles) {
+    if (uni) adj_pass_b_kernel<true, true><<<all, 128, 0, stream>>>(p, q, none, whole, 0);
+    else adj_pass_b_kernel<false, true><<<all, 128, 0, stream>>>(p, q, none, whole, 0);
   } else {
-    adj_pass_a_kernel<false><<<cells, 128, 0, stream>>>(p, q);
-    if (poles) adj_pass_b_kernel<false, true><<<cells, 128, 0, stream>>>(p, q);
-    else adj_pass_b_kernel<false, false><<<cells, 128, 0, stream>>>(p, q);
+    if (uni) adj_pass_b_kernel<true, false><<<blocks(shell_b, first_b), 128, 0, stream>>>(p, q, box_b, shell_b, first_b);
+    else adj_pass_b_kernel<false, false><<<blocks(shell_b, first_b), 128, 0, stream>>>(p, q, box_b, shell_b, first_b);
   }
-  adj_pass_c_kernel<<<cells, 128, 0, stream>>>(p, q);
+  // without magnetic loss pass C has work in the slabs only
+  bool unit = true;
+  for (int c = 0; c < 3; ++c) unit = unit && !p.hdecay[c] && p.hdecay_u[c] == 1.0f;
+  if (unit && !p.cpml) return static_cast<int>(cudaGetLastError());
+  const Shell shell_c = unit ? shell_of(p, plain_box(p, 0, 0, 2)) : whole;
+  adj_pass_c_kernel<<<blocks(shell_c, 0), 128, 0, stream>>>(p, q, shell_c);
   return static_cast<int>(cudaGetLastError());
 }
 
