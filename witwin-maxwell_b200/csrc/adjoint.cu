@@ -199,12 +199,7 @@ __device__ __forceinline__ void pass_a_cell(const StepParams& p, const AdjParams
 
 // ---- pass B: gE = de gE' - C_E^T g(d_H); adjoint E psi; design gradient ----
 // kPoles: the scene has ADE poles (their transpose is compiled only then: in
-// the per-component loop it slows the pole-free kernel by a third).  The
-// pole-free kernel runs twelve 128-thread CTAs per SM (40 registers, no
-// spills): the pass is latency-bound, and 48 resident warps against 32 at 64
-// registers took the backward of the 160x160x96 design workload from 910 to
-// 782 ms.  The pole kernel spills at that budget and runs five CTAs per SM
-// (at most 102 registers, 70-72 used).
+// the per-component loop it slows the pole-free kernel by a third).
 template <bool kUniform, bool kPoles>
 __device__ __forceinline__ void pass_b_cell(const StepParams& p, const AdjParams& q, int i, int j, int k) {
   {
@@ -404,8 +399,9 @@ __device__ __forceinline__ bool shell_cell(const StepParams& p, const Shell& s, 
 // multiples of four), every one a plain cell: a thread takes four consecutive z
 // cells, so that a neighbour read is one 16-byte load for the four (and one value
 // for the shifted cell).  Both passes are bound by instruction issue and L2 latency:
-// one cell per thread took 97 and 137 us per step of the 160 x 160 x 96 design, whose
-// state stays in L2.  The cells around the box (slabs, faces) stay one per thread.
+// one cell per thread takes 97 and 137 us over the 160 x 160 x 96 design, 68 and 90
+// over the half of its cells outside the box; four take 22 and 25 over the other half.
+// The cells around the box (slabs, faces) stay one per thread.
 struct Box {
   int x0, x1, y0, y1, k0, k1;
 };
