@@ -66,6 +66,24 @@ def test_tiles_agree_with_each_other_and_with_the_warp_kernel(cells, pml, bounda
     assert np.sqrt(num) <= TOL
 
 
+@pytest.mark.parametrize("rows", [1, 2, 3, 4, 5, 6, 7])
+def test_lanes_past_the_last_quad_leave_the_fields_alone(rows):
+    """Tiles whose (rows + 1) * 6 quads end inside a warp: the lanes past the last quad
+    repeat it and may write nothing.  TFSF faces put H terms (added to the H that the
+    ring holds) on rows of every place in a tile, the last one among them."""
+    wm = load_package()
+    cs = _scene(wm, (13, 14, 22), 2, (1,) * 6, tfsf=True)
+    assert (rows + 1) * ((cs.nodes[2] + 3) // 4) % 32 != 0
+    _, one = _run(wm, cs, (11, 15, 3))
+    _, got = _run(wm, cs, (11, rows, 4))
+    _, ref = _run(wm, cs, (2, 1, 0))
+    for n in FIELDS:
+        np.testing.assert_array_equal(got[n], one[n], err_msg=n)
+        assert np.linalg.norm(ref[n]) > 0
+    num = sum(np.linalg.norm(got[n].astype(np.float64) - ref[n]) ** 2 / np.linalg.norm(ref[n].astype(np.float64)) ** 2 for n in FIELDS)
+    assert np.sqrt(num) <= TOL
+
+
 def test_rows_beyond_a_tile_run_another_kernel():
     wm = load_package()
     solver = wm.solver.B200FDTD(_scene(wm, (8, 8, 512), 2, (1,) * 6)).init_field()

@@ -245,7 +245,7 @@ __device__ __forceinline__ void copy_march(const StepParams& p, const Tile& t, f
 // Flags of a thread's quad (and, or-ed over the warp, of the warp).
 constexpr unsigned kZLast = 7u, kZFirst = 1u << 3, kValid = 1u << 4, kOwn = 1u << 5, kYFace = 1u << 6, kYLast = 1u << 7,
                    kYPec = 1u << 8, kYSlabH = 1u << 9, kYSlabE = 1u << 10, kZSlabH = 1u << 11, kZSlabE = 1u << 12,
-                   kWarpZFace = 1u << 13, kWarpECoef = 1u << 14, kWarpHCoef = 1u << 15;
+                   kWarpZFace = 1u << 13, kWarpECoef = 1u << 14, kWarpHCoef = 1u << 15, kItem = 1u << 16;
 constexpr unsigned kYSlab = kYSlabH | kYSlabE, kZSlab = kZSlabH | kZSlabE;
 
 // Offset of a row's y-slab psi (row 0 of the slab where the row has none).
@@ -469,7 +469,10 @@ __device__ __forceinline__ void quad_march(const StepParams& p, const QuadTerms&
         fill4(hz, 0.f);
       }
       if (tmask & terms.h_bits) quad_terms(terms, tmask & terms.h_bits, 3, n, i, j, k, hx, hy, hz);
-      if (own) {
+      // One writer for each quad of the ring: a thread that repeats the last item
+      // reads the same H^{n-1/2} and, writing too, could be read by the item's own
+      // thread before that has loaded it (the lanes of a warp need not run together).
+      if (own && (fl & kItem)) {
         st4(hown, hx);
         st4(hown + h_pitch, hy);
         st4(hown + 2 * h_pitch, hz);
@@ -647,7 +650,8 @@ __global__ void __launch_bounds__(quad_max_threads(kCpml), 1)
   // ---- the thread's quad ----
   // Items are the quads of rows j0 - 1 .. j0 + TY - 1; the first and last few
   // quads of each row (z faces and slabs) come first, so that their code runs in
-  // a few warps only.  Threads past the last item repeat it and store nothing.
+  // a few warps only.  Threads past the last item repeat it and store nothing,
+  // neither to memory nor to the ring.
   const int rows = shape.TY + 1, ns = shape.nlo + shape.nhi, items = rows * Q;
   const int item = min(static_cast<int>(threadIdx.x), items - 1);
   int r, col;
@@ -671,6 +675,7 @@ __global__ void __launch_bounds__(quad_max_threads(kCpml), 1)
   unsigned fl = k <= NZ - 1 && k + 4 > NZ - 1 ? NZ - 1 - k : 4;  // kZLast: cell NZ - 1 of the quad (4: not here)
   if (k == 0) fl |= kZFirst;
   if (valid) fl |= kValid;
+  if (static_cast<int>(threadIdx.x) < items) fl |= kItem;
   if (eitem) fl |= kOwn;
   if (j == 0 || j == NY - 1) fl |= kYFace;
   if (j == NY - 1) fl |= kYLast;
