@@ -94,6 +94,47 @@ def test_rows_beyond_a_tile_run_another_kernel():
     solver.close()
 
 
+def test_two_threads_step_tiles_of_different_sizes():
+    """Two solvers of one kernel, one on the largest tile and one on the smallest, stepped
+    on a stream and a thread each: neither makes the other's launch fail, and both give
+    the fields of stepping alone."""
+    import threading
+
+    import torch
+
+    wm = load_package()
+    cases = [((12, 40, 120), (11, 18, 13)), ((12, 9, 10), (11, 1, 13))]  # 190 and 3 KB of shared memory
+    scenes = [_scene(wm, cells, 3, (1,) * 6) for cells, _ in cases]
+    want = [_run(wm, cs, launch)[1] for cs, (_, launch) in zip(scenes, cases)]
+    got, errors = [None, None], []
+
+    def work(k):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                solver = wm.solver.B200FDTD(scenes[k]).init_field()
+                solver.set_launch(*cases[k][1])
+                solver.checkpoint_save(0)
+                start.wait()
+                for _ in range(400):
+                    solver.checkpoint_load(0)
+                    solver.step_range(0, STEPS)
+                got[k] = {n: solver.field(n).cpu().numpy() for n in FIELDS}
+                solver.close()
+        except Exception as err:  # noqa: BLE001 (reported below)
+            errors.append(err)
+
+    start = threading.Barrier(2, timeout=60)
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for k in range(2):
+        for n in FIELDS:
+            np.testing.assert_array_equal(got[k][n], want[k][n])
+
+
 def test_a_wait_that_runs_out_is_reported():
     wm = load_package()
     solver = wm.solver.B200FDTD(_scene(wm, (24, 20, 18), 4, (1,) * 6)).init_field()

@@ -2632,6 +2632,8 @@ int fdtd_engine_finalize(fdtd_engine* h) {
       if (err == 0)
         err = launch_quad_ztable(h->eb[2], h->ec[2], h->eik[2], h->inv_e[2], h->NZ, lo, hi, h->P, h->d_ztab_e, h->stream);
       if (err != 0) return cuda_fail(static_cast<cudaError_t>(err), "quad_ztable_kernel launch");
+      err = prepare_quad_step(h->cpml, has_coef(h), h->uniform_grid);
+      if (err != 0) return cuda_fail(static_cast<cudaError_t>(err), "shared memory of quad_step_kernel");
     }
     CUDA_TRY(pool_alloc(&h->d_status, sizeof(int), h->stream));
     CUDA_TRY(cudaMemsetAsync(h->d_status, 0, sizeof(int), h->stream));

@@ -799,31 +799,28 @@ int launch_quad_ztable(const float* b, const float* c, const float* ik, const fl
   return static_cast<int>(cudaGetLastError());
 }
 
+namespace {
+using QuadKernel = void (*)(StepParams, QuadTerms, QuadShape, int);
+template <bool kCpml, bool kCoef>
+QuadKernel quad_kernel_of(bool uni) {
+  return uni ? quad_step_kernel<kCpml, kCoef, true> : quad_step_kernel<kCpml, kCoef, false>;
+}
+QuadKernel quad_kernel_of(bool cpml, bool coef, bool uni) {
+  if (cpml) return coef ? quad_kernel_of<true, true>(uni) : quad_kernel_of<true, false>(uni);
+  return coef ? quad_kernel_of<false, true>(uni) : quad_kernel_of<false, false>(uni);
+}
+}  // namespace
+
+int prepare_quad_step(bool cpml, bool coef, bool uni) {
+  return static_cast<int>(cudaFuncSetAttribute(quad_kernel_of(cpml, coef, uni),
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(kQuadMaxSmem)));
+}
+
 int launch_quad_step(const StepParams& p, const QuadTerms& terms, const QuadShape& s, int n, dim3 grid,
                      bool coef, bool uni, cudaStream_t stream) {
-  const size_t bytes = quad_smem_bytes(s.TY, p.P, p.SZ);
-  // dynamic shared memory beyond 48 KB is opted into per kernel and device
-  // context; the call is cheap, needs no stream and is allowed under capture
-#define FDTD_QUAD(CPML, COEF, UNI)                                                                           \
-  do {                                                                                                       \
-    auto kern = quad_step_kernel<CPML, COEF, UNI>;                                                           \
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
-                                               static_cast<int>(bytes));                                    \
-    if (e != cudaSuccess) return static_cast<int>(e);                                                        \
-    kern<<<grid, s.threads, bytes, stream>>>(p, terms, s, n);                                                \
-  } while (0)
-  if (p.cpml) {
-    if (coef && uni) FDTD_QUAD(true, true, true);
-    else if (coef) FDTD_QUAD(true, true, false);
-    else if (uni) FDTD_QUAD(true, false, true);
-    else FDTD_QUAD(true, false, false);
-  } else {
-    if (coef && uni) FDTD_QUAD(false, true, true);
-    else if (coef) FDTD_QUAD(false, true, false);
-    else if (uni) FDTD_QUAD(false, false, true);
-    else FDTD_QUAD(false, false, false);
-  }
-#undef FDTD_QUAD
+  const QuadKernel kern = quad_kernel_of(p.cpml != 0, coef, uni);
+  kern<<<grid, s.threads, quad_smem_bytes(s.TY, p.P, p.SZ), stream>>>(p, terms, s, n);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -35,6 +35,11 @@ struct QuadTerms {
 
 // SZ: floats of a z-slab psi row (0 without z slabs).
 size_t quad_smem_bytes(int TY, int P, int SZ);
+// Once per engine, on its device, before its first launch: opts the engine's kernel in
+// to the largest tile's shared memory.  The limit belongs to the function and the
+// device, which other engines and threads share, so it is the same for every engine:
+// set to the launch's own size, it could be lowered by another thread in between.
+int prepare_quad_step(bool cpml, bool coef, bool uni);
 int launch_quad_step(const StepParams& p, const QuadTerms& terms, const QuadShape& s, int n, dim3 grid, bool coef,
                      bool uni, cudaStream_t stream);
 // Class table [chunk][NY][P / 4] of the current chunk length p.CX.
