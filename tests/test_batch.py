@@ -78,6 +78,61 @@ def test_batch_autotune_keeps_results():
         s.close()
 
 
+def _closed_scene(wm, cells, n_sources, steps, pml=0):
+    sc = wm.Scene(cells=cells, spacing=25e-9, pml_cells=pml, boundary=(1,) * 6 if pml else (4,) * 6)
+    for n in range(n_sources):
+        at = (3 + n % 5 * 3, 4 + n // 5 * 3, cells[2] // 2)
+        sc.sources.append(wm.PointDipole(at, "Ez", wm.GaussianPulse(300e12, 100e12, delay=0.5e-15), width=25e-9))
+    sc.monitors.append(wm.PointMonitor("probe", tuple(c // 2 for c in cells), frequencies=(250e12, 300e12)))
+    return wm.compile_scene(sc, steps)
+
+
+def test_batch_autotune_gives_equal_scenes_the_same_launch():
+    """Engines of one shape take the tuned tile as it is, its rows included."""
+    wm = load_package()
+    solvers = [wm.solver.B200FDTD(_closed_scene(wm, (96, 96, 96), 1, 64, pml=8)).init_field() for _ in range(3)]
+    batch = wm.solver.B200Batch(solvers)
+    batch.autotune()
+    launches = [s.get_launch() for s in solvers]
+    assert launches[0][0] == 11 and launches[0][1] > 1
+    assert launches == [launches[0]] * 3
+    batch.close()
+    for s in solvers:
+        s.close()
+
+
+@pytest.mark.parametrize("shapes", [
+    [((20, 20, 24), 24), ((20, 20, 24), 25)],    # one size class: 24 injection terms, and more than the quad tile takes
+    [((20, 20, 511), 1), ((20, 20, 512), 1)],    # 512 z nodes, and one more
+    [((20, 30, 40), 1), ((21, 24, 42), 1)],      # other row lengths and counts
+])
+def test_batch_autotune_of_a_mixed_class(shapes):
+    wm = load_package()
+    steps = 32
+    compiled = [_closed_scene(wm, cells, n, steps) for cells, n in shapes]
+    ref = []
+    for cs in compiled:
+        s = wm.solver.B200FDTD(cs).init_field()
+        s.step_range(0, steps)
+        ref.append(_state(s))
+        s.close()
+    solvers = [wm.solver.B200FDTD(cs).init_field() for cs in compiled]
+    batch = wm.solver.B200Batch(solvers)
+    batch.autotune()
+    batch.step_range(0, steps)
+    for s, (rf, _) in zip(solvers, ref):
+        f, _ = _state(s)
+        for group in (FIELDS[:3], FIELDS[3:]):
+            # another kernel rounds up to three products of a cell differently each step (Hz
+            # of z dipoles is nothing but such rounding: E and H as wholes)
+            got, want = (np.concatenate([x[n].ravel() for n in group]).astype(np.float64) for x in (f, rf))
+            assert np.linalg.norm(want) > 0
+            assert np.linalg.norm(got - want) <= 3 * steps * 2.0 ** -24 * np.linalg.norm(want)
+    batch.close()
+    for s in solvers:
+        s.close()
+
+
 def test_batch_rejects_mismatched_sample_blocks():
     wm = load_package()
     compiled = [wm.compile_scene(sc, 10) for sc in _scenes(wm)[:2]]
