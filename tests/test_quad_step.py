@@ -84,6 +84,24 @@ def test_lanes_past_the_last_quad_leave_the_fields_alone(rows):
     assert np.sqrt(num) <= TOL
 
 
+@pytest.mark.parametrize("pml,boundary,other", [(0, (4,) * 6, 10), (3, (1,) * 6, 2), (3, (2, 2, 2, 2, 1, 1), 2)])
+def test_terms_beyond_the_table_run_another_kernel(pml, boundary, other):
+    """24 injection terms fit the kernel's table; with 25 the engine runs the kernel that
+    it would run without this one."""
+    wm = load_package()
+    for n_terms, variant in ((24, 11), (25, other)):
+        sc = wm.Scene(cells=(18, 17, 19), spacing=25e-9, pml_cells=pml, boundary=boundary)
+        for n in range(n_terms):
+            pulse = wm.GaussianPulse(300e12, 100e12, delay=0.5e-15)
+            sc.sources.append(wm.PointDipole((4 + n % 5 * 2, 4 + n // 5 * 2, 8), "E" + "xyz"[n % 3], pulse, width=25e-9))
+        cs = wm.compile_scene(sc, STEPS)
+        picked, got = _run(wm, cs, None)
+        assert picked == variant
+        _, ref = _run(wm, cs, (2, 1, 0))
+        num = sum(np.linalg.norm(got[n].astype(np.float64) - ref[n]) ** 2 / np.linalg.norm(ref[n].astype(np.float64)) ** 2 for n in FIELDS)
+        assert np.sqrt(num) <= TOL
+
+
 def test_rows_beyond_a_tile_run_another_kernel():
     wm = load_package()
     solver = wm.solver.B200FDTD(_scene(wm, (8, 8, 512), 2, (1,) * 6)).init_field()

@@ -1139,6 +1139,12 @@ void default_tiles(fdtd_engine* h) {
   h->CX = CX;
 }
 
+// Default variant of an engine that the quad-tile kernel does not take: the row-tile
+// kernel without CPML and wrapped or PMC faces, else the warp kernel.
+int other_variant(const fdtd_engine* h) {
+  return !h->wrap && !h->cpml && !h->pmc ? kTileVariant : kDefaultVariant;
+}
+
 bool quad_runs(const fdtd_engine* h);
 
 // Task grid of the warp kernel (and of the other kernels with its layout).
@@ -1708,11 +1714,9 @@ int fdtd_engine_create(const fdtd_grid_desc* desc, void* stream, fdtd_engine** o
     fdtd_engine_destroy(h);
     return rc;
   }
-  // The quad-tile kernel runs where a row fits its CTA and no face is PMC.  Beside
-  // it stay the row-tile kernel (longer rows without CPML or wrapped faces) and
-  // the warp kernel.
-  if (!h->pmc && h->P <= kQuadMaxPitch) h->variant = kQuadVariant;
-  else if (!h->wrap && !h->cpml && !h->pmc) h->variant = kTileVariant;
+  // The quad-tile kernel runs where a row fits its CTA and no face is PMC (finalize
+  // looks at the numbers of poles and injection terms).
+  h->variant = !h->pmc && h->P <= kQuadMaxPitch ? kQuadVariant : other_variant(h);
   default_tiles(h);
   *out = h;
   return 0;
@@ -2461,8 +2465,8 @@ int fdtd_engine_finalize(fdtd_engine* h) {
   if (h->variant == kQuadVariant && (h->poles.size() > static_cast<size_t>(kAdeMaxPoles) ||
                                      h->terms.size() > static_cast<size_t>(kQuadMaxTerms))) {
     // more poles than the ADE pass takes, or more injection terms than the
-    // quad-tile kernel's table: the warp kernel runs
-    h->variant = kDefaultVariant;
+    // quad-tile kernel's table: the default of the engines that it does not take
+    h->variant = other_variant(h);
     default_tiles(h);
   }
   if (!h->poles.empty() && h->poles.size() <= static_cast<size_t>(kAdeMaxPoles)) {
