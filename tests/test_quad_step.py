@@ -102,6 +102,29 @@ def test_terms_beyond_the_table_run_another_kernel(pml, boundary, other):
         assert np.sqrt(num) <= TOL
 
 
+def test_many_terms_on_a_row_shorten_the_chunks():
+    """Sources over the same cells of a closed box: shorter chunks (a CTA that holds them
+    all ends last) and the fields of the longer ones; a launch that is set stays."""
+    wm = load_package()
+    launches, fields = [], []
+    for n_terms, launch in ((1, None), (12, None), (12, (11, 0, 40))):
+        sc = wm.Scene(cells=(120, 64, 64), spacing=25e-9, boundary=(4,) * 6)
+        for n in range(n_terms):
+            pulse = wm.GaussianPulse(300e12, 100e12, delay=0.5e-15)
+            sc.sources.append(wm.PointDipole((60 + n % 3, 32 + n // 3, 32), "E" + "xyz"[n % 3], pulse, width=25e-9))
+        solver = wm.solver.B200FDTD(wm.compile_scene(sc, STEPS)).init_field()
+        if launch:
+            solver.set_launch(*launch)
+        launches.append(solver.get_launch())
+        solver.step_range(0, STEPS)
+        fields.append({n: solver.field(n).cpu().numpy() for n in FIELDS})
+        solver.close()
+    assert launches[0][0] == launches[1][0] == 11 and launches[2][2] == 40
+    assert launches[1][2] < launches[0][2]
+    for n in FIELDS:
+        np.testing.assert_array_equal(fields[1][n], fields[2][n])
+
+
 def test_rows_beyond_a_tile_run_another_kernel():
     wm = load_package()
     solver = wm.solver.B200FDTD(_scene(wm, (8, 8, 512), 2, (1,) * 6)).init_field()

@@ -771,6 +771,7 @@ struct fdtd_engine {
   // exchange, tile_kernel.cu); 11 = quad-tile kernel (four z cells per thread,
   // bulk-copied planes, quad_kernel.cu).
   int variant = kDefaultVariant;
+  bool launch_set = false;  // by fdtd_engine_set_launch
   int pf_dist = kDefaultPrefetch;
   int cur = 0;  // index of the buffer holding the current state
   float* E[2][3] = {};
@@ -1052,6 +1053,22 @@ int warp_chunk(const fdtd_engine* h) {
   return static_cast<int>(std::max<int64_t>(4, (h->NX + want_chunks - 1) / want_chunks));
 }
 
+// The most (term, plane) pairs of a row's injection terms in a chunk of `planes`
+// planes; 0 where no row holds more than two terms.
+int term_planes(const fdtd_engine* h, int planes) {
+  int most = 0;
+  for (const InjectionTerm& a : h->terms) {  // the fullest row is some term's first
+    int terms = 0, sum = 0;
+    for (const InjectionTerm& t : h->terms)
+      if (a.j0 >= t.j0 && a.j0 < t.j1) {
+        ++terms;
+        sum += std::min(planes, t.i1 - t.i0);
+      }
+    if (terms > 2) most = std::max(most, sum);
+  }
+  return most;
+}
+
 // Tile of the quad-tile kernel: TY rows, CX planes (ty, cx > 0 fix TY and CX).
 // Picks the smallest modelled step time; its constants come from sweeps of TY and
 // CX (B200):
@@ -1065,7 +1082,11 @@ int warp_chunk(const fdtd_engine* h) {
 //   whole one (257 x 257 x 193, z slabs only: 265 us at 1.9 and 7.0 rounds, 301 at
 //   2.1; 182 x 212 x 158: 56 us at TY 7, CX 10, 70 at 8, 14).  CTAs in a slab take
 //   about twice as long: the tail is 1.5 CTAs, and a single round ends with its
-//   slowest CTA (193 x 193 x 161, TY 13: 105 us at 5 planes, 133 at 22).
+//   slowest CTA (193 x 193 x 161, TY 13: 105 us at 5 planes, 133 at 22);
+// - without CPML the chunks are long, and a CTA whose rows hold many injection terms
+//   ends last: 0.6 us a term and plane (24 dipoles over the same cells of 257^3: 426 us
+//   at 29 planes, 180 at 6; 8 of them: 211 and 144).  One or two cost less than
+//   shorter chunks do (193^3, one: 63.5 us at 13 planes, 65.5 at 10).
 void default_quad(fdtd_engine* h, int ty, int cx) {
   const int Q = h->P / 4;
   double best = 1e300;
@@ -1078,6 +1099,7 @@ void default_quad(fdtd_engine* h, int ty, int cx) {
     s.nlo = Q;
     s.nhi = 0;
   }
+  std::vector<int> crowd(h->cpml ? 0 : h->NX + 1, -1);  // term_planes of a chunk length
   for (int TY = ty > 0 ? ty : 1; TY <= (ty > 0 ? ty : h->NY); ++TY) {
     s.TY = TY;
     s.threads = ((TY + 1) * Q + 31) / 32 * 32 + 32;
@@ -1097,7 +1119,12 @@ void default_quad(fdtd_engine* h, int ty, int cx) {
       const double plane = std::max(lat, resident * (TY * bytes_cell + 36.0) * h->P / (one ? 42.0 : 50.0));
       const double cta = (CX + (chunks > 1 ? 1.0 : 0.0) + (one ? 1.5 : 0.0)) * plane;
       const double waves = blocks / (148.0 * occ);
-      const double cost = cta * (!xy ? std::ceil(waves) : waves <= 1.0 ? 2.0 : waves + 1.5);
+      double cost = cta * (!xy ? std::ceil(waves) : waves <= 1.0 ? 2.0 : waves + 1.5);
+      if (!h->cpml) {
+        int& n = crowd[std::min(CX, h->NX)];
+        if (n < 0) n = term_planes(h, CX + 1);
+        if (n > 0) cost = std::max(cost, cta + 600.0 * n);
+      }
       if (cost < best) {
         best = cost;
         h->quad = s;
@@ -2468,6 +2495,8 @@ int fdtd_engine_finalize(fdtd_engine* h) {
     // quad-tile kernel's table: the default of the engines that it does not take
     h->variant = other_variant(h);
     default_tiles(h);
+  } else if (h->variant == kQuadVariant && !h->launch_set) {
+    default_tiles(h);  // with the injection terms
   }
   if (!h->poles.empty() && h->poles.size() <= static_cast<size_t>(kAdeMaxPoles)) {
     // ADE pass: the pole table, and tiles over the z range of each (i, j) row
@@ -3017,6 +3046,7 @@ int fdtd_engine_set_launch(fdtd_engine* h, int variant, int tile_rows, int chunk
     return fail(FDTD_ERR_UNSUPPORTED, "the quad-tile kernel takes up to 512 z nodes and 24 injection terms");
   if (h->nl_general >= 0 && !h->poles.empty() && variant > 3 && variant < kTileVariant)
     return fail(FDTD_ERR_UNSUPPORTED, "nonlinear media with poles run launch variants 1-3, 10 and 11");
+  h->launch_set = true;
   if (variant == kQuadVariant) {
     // the only tile with rows: an explicit height has to fit a CTA
     const QuadShape keep = h->quad;
