@@ -49,11 +49,11 @@ extern "C" {
 /* Last error message of the calling thread (engine-independent). */
 const char* fdtd_last_error(void);
 /* Library version string. */
-/* The engines of a device take their arrays from one memory pool, which keeps up to
- * 4 GiB of what destroyed engines gave back.  This returns all but keep_bytes of the
- * unused memory to the current device (it waits for the device first). */
-int fdtd_release_memory(uint64_t keep_bytes);
 const char* fdtd_version(void);
+/* The engines of a device that were created without an allocator take their arrays from
+ * one memory pool, which keeps nothing of what a destroyed engine gave back.  This
+ * waits for the device and returns all but keep_bytes of what the pool holds unused. */
+int fdtd_release_memory(uint64_t keep_bytes);
 
 /* ------------------------------------------------------------------------ */
 /* 1. Fused step engine                                                       */
@@ -74,6 +74,16 @@ typedef struct {
 /* Create an engine on the current CUDA device.  Replaces FDTD.init_field,
  * witwin/maxwell/fdtd/runtime/stepping.py:1624-1654 (field allocation). */
 int fdtd_engine_create(const fdtd_grid_desc* desc, void* stream, fdtd_engine** out);
+/* The same with the caller's device memory: alloc returns at least `bytes` of `device`,
+ * 256-byte aligned, for use in the order of `stream` (the engine's), or NULL; release
+ * takes such a pointer back, in the same order.  They are called by the threads that
+ * call the engine, until it (and a batch that it is the first engine of) is destroyed,
+ * and never while stepping.  A caching allocator keeps building and destroying engines
+ * cheap and lets the caller's other arrays use what a destroyed engine held. */
+typedef void* (*fdtd_alloc_fn)(size_t bytes, int device, void* stream, void* user);
+typedef void (*fdtd_free_fn)(void* memory, void* user);
+int fdtd_engine_create_with(const fdtd_grid_desc* desc, void* stream, fdtd_alloc_fn alloc, fdtd_free_fn release,
+                            void* user, fdtd_engine** out);
 int fdtd_engine_destroy(fdtd_engine* h);
 
 /* Field storage of the engine's state: FDTD_STORE_F32 (default, exact FP32

@@ -36,10 +36,14 @@ class FdtdGridDesc(ctypes.Structure):
     ]
 
 
+ALLOC_FN = ctypes.CFUNCTYPE(_vp, ctypes.c_size_t, _i, _vp, _vp)
+FREE_FN = ctypes.CFUNCTYPE(None, _vp, _vp)
+
 _SIGNATURES = {
     "fdtd_last_error": ([], ctypes.c_char_p),
     "fdtd_version": ([], ctypes.c_char_p),
     "fdtd_engine_create": ([ctypes.POINTER(FdtdGridDesc), _vp, ctypes.POINTER(_vp)], _i),
+    "fdtd_engine_create_with": ([ctypes.POINTER(FdtdGridDesc), _vp, ALLOC_FN, FREE_FN, _vp, ctypes.POINTER(_vp)], _i),
     "fdtd_engine_destroy": ([_vp], _i),
     "fdtd_bloch_create": ([_vp, _vp, ctypes.POINTER(_f), ctypes.POINTER(_f), ctypes.POINTER(_vp)], _i),
     "fdtd_bloch_destroy": ([_vp], _i),

@@ -81,14 +81,14 @@ int cuda_fail(cudaError_t err, const char* what) {
     if (err__ != cudaSuccess) return cuda_fail(err__, #expr); \
   } while (0)
 
-// Device memory of the engines: one memory pool per device, from which an engine
-// takes its arrays in stream order.  Creating an engine makes about a hundred
-// allocations and destroying it as many frees; cudaMalloc and cudaFree take 50 us to
-// milliseconds each and wait for the device (65^3: 11 of a 20 ms solve; one
-// iteration of the 160 x 160 x 96 design with 16 checkpoints: 200 to 700 ms).
-// What a destroyed engine gave back stays in the pool up to kPoolKeep, and goes back
-// to the device beyond it at the next synchronisation.
-constexpr uint64_t kPoolKeep = 4ull << 30;
+// Device memory of an engine: the caller's allocator (fdtd_engine_create_with), else
+// one memory pool per device.  Creating an engine makes about a hundred allocations
+// and destroying it as many frees; cudaMalloc and cudaFree take 50 us to milliseconds
+// each and wait for the device (65^3: 11 of a 20 ms solve; one iteration of the 160 x
+// 160 x 96 design with 16 checkpoints: 200 to 700 ms), so a program that makes engines
+// again and again passes the allocator that it keeps its own arrays in.  The pool
+// keeps nothing: what a destroyed engine gave back is the device's again, since no
+// other allocator could ask the pool for it.
 constexpr int kMaxDevices = 64;
 
 cudaError_t device_pool(cudaMemPool_t* out) {
@@ -105,46 +105,61 @@ cudaError_t device_pool(cudaMemPool_t* out) {
     props.handleTypes = cudaMemHandleTypeNone;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = dev;
-    cudaMemPool_t pool = nullptr;
-    err = cudaMemPoolCreate(&pool, &props);
-    if (err != cudaSuccess) return err;
-    uint64_t keep = kPoolKeep;
-    err = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    err = cudaMemPoolCreate(&pools[dev], &props);  // its release threshold is 0
     if (err != cudaSuccess) {
-      cudaMemPoolDestroy(pool);
+      pools[dev] = nullptr;
       return err;
     }
-    pools[dev] = pool;
   }
   *out = pools[dev];
   return cudaSuccess;
 }
 
-template <typename T>
-cudaError_t pool_alloc(T** out, size_t bytes, cudaStream_t stream) {
-  *out = nullptr;
-  cudaMemPool_t pool = nullptr;
-  cudaError_t err = device_pool(&pool);
-  if (err != cudaSuccess) return err;
-  void* p = nullptr;
-  err = cudaMallocFromPoolAsync(&p, std::max<size_t>(bytes, 1), pool, stream);
-  if (err == cudaErrorMemoryAllocation) {
-    // memory that other engines gave back on streams not yet synchronised
-    cudaGetLastError();
-    cudaDeviceSynchronize();
-    cudaMemPoolTrimTo(pool, 0);
-    err = cudaMallocFromPoolAsync(&p, std::max<size_t>(bytes, 1), pool, stream);
-  }
-  if (err == cudaSuccess) *out = static_cast<T*>(p);
-  return err;
-}
+// Allocation and release in the order of `stream`, the engine's own, which stays the
+// same for its life.
+struct DeviceMemory {
+  fdtd_alloc_fn caller_alloc = nullptr;
+  fdtd_free_fn caller_free = nullptr;
+  void* user = nullptr;
 
-void pool_free(void* p, cudaStream_t stream) {
-  if (p && cudaFreeAsync(p, stream) != cudaSuccess) {
-    cudaGetLastError();  // the caller's stream is gone: free in device order
-    cudaFree(p);
+  template <typename T>
+  cudaError_t alloc(T** out, size_t bytes, cudaStream_t stream) const {
+    *out = nullptr;
+    bytes = std::max<size_t>(bytes, 1);
+    void* p = nullptr;
+    if (caller_alloc) {
+      int dev = 0;
+      const cudaError_t err = cudaGetDevice(&dev);
+      if (err != cudaSuccess) return err;
+      p = caller_alloc(bytes, dev, stream, user);
+      *out = static_cast<T*>(p);
+      return p ? cudaSuccess : cudaErrorMemoryAllocation;
+    }
+    cudaMemPool_t pool = nullptr;
+    cudaError_t err = device_pool(&pool);
+    if (err != cudaSuccess) return err;
+    err = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
+    if (err == cudaErrorMemoryAllocation) {
+      // memory that other engines gave back on streams not yet synchronised
+      cudaGetLastError();
+      cudaDeviceSynchronize();
+      cudaMemPoolTrimTo(pool, 0);
+      err = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
+    }
+    if (err == cudaSuccess) *out = static_cast<T*>(p);
+    return err;
   }
-}
+
+  void free(void* p, cudaStream_t stream) const {
+    if (!p) return;
+    if (caller_free) {
+      caller_free(p, user);
+    } else if (cudaFreeAsync(p, stream) != cudaSuccess) {
+      cudaGetLastError();  // the caller's stream is gone: free in device order
+      cudaFree(p);
+    }
+  }
+};
 
 int axis_a(int comp) { return comp == 0 ? 1 : 0; }
 int axis_b(int comp) { return comp == 2 ? 1 : 2; }
@@ -794,6 +809,7 @@ struct fdtd_engine {
   float inv_e_u[3] = {0, 0, 0}, inv_h_u[3] = {0, 0, 0};
   std::vector<InjectionTerm> terms;
   std::vector<ShiftedHost> shifted;
+  DeviceMemory mem;
   std::vector<float*> owned;
   std::vector<PoleHost> poles;
   std::vector<SampleRegion> regions;
@@ -863,7 +879,7 @@ int dev_alloc(fdtd_engine* h, float** out, size_t n) {
     *out = nullptr;
     return 0;
   }
-  CUDA_TRY(pool_alloc(out, n * sizeof(float), h->stream));
+  CUDA_TRY(h->mem.alloc(out, n * sizeof(float), h->stream));
   CUDA_TRY(cudaMemsetAsync(*out, 0, n * sizeof(float), h->stream));
   h->owned.push_back(*out);
   return 0;
@@ -917,13 +933,13 @@ int background_value(fdtd_engine* h, int comp, const float* arr, float* out) {
   int ext[3];
   comp_extent(comp, h->NX, h->NY, h->NZ, ext);
   float* d = nullptr;
-  CUDA_TRY(pool_alloc(&d, sizeof(float) * kSamples, h->stream));
+  CUDA_TRY(h->mem.alloc(&d, sizeof(float) * kSamples, h->stream));
   coef_sample_kernel<<<kSamples / 256, 256, 0, h->stream>>>(arr, h->NY, h->P, ext[0], ext[1], ext[2], kSamples, d);
   std::vector<float> v(kSamples);
   cudaError_t err = cudaGetLastError();
   if (err == cudaSuccess) err = cudaMemcpyAsync(v.data(), d, sizeof(float) * kSamples, cudaMemcpyDeviceToHost, h->stream);
   if (err == cudaSuccess) err = cudaStreamSynchronize(h->stream);
-  pool_free(d, h->stream);
+  h->mem.free(d, h->stream);
   if (err != cudaSuccess) return cuda_fail(err, "coefficient background sample");
   std::sort(v.begin(), v.end());
   float best = v[0];
@@ -1551,10 +1567,10 @@ int flush_samples(fdtd_engine* h) {
 
 template <typename T>
 int upload_vec(fdtd_engine* h, T** dptr, const std::vector<T>& v) {
-  if (*dptr) pool_free(*dptr, h->stream);
+  if (*dptr) h->mem.free(*dptr, h->stream);
   *dptr = nullptr;
   if (v.empty()) return 0;
-  CUDA_TRY(pool_alloc(dptr, v.size() * sizeof(T), h->stream));
+  CUDA_TRY(h->mem.alloc(dptr, v.size() * sizeof(T), h->stream));
   CUDA_TRY(cudaMemcpyAsync(*dptr, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, h->stream));
   return 0;
 }
@@ -1575,7 +1591,7 @@ void build_plane_csr(int NX, const std::vector<T>& items, std::vector<int>& ptr,
 int upload_ints(fdtd_engine* h, const std::vector<int>& v, const int** out) {
   int* d = nullptr;
   const size_t n = std::max<size_t>(v.size(), 1);
-  CUDA_TRY(pool_alloc(&d, n * sizeof(int), h->stream));
+  CUDA_TRY(h->mem.alloc(&d, n * sizeof(int), h->stream));
   CUDA_TRY(cudaMemsetAsync(d, 0, n * sizeof(int), h->stream));
   if (!v.empty()) CUDA_TRY(cudaMemcpyAsync(d, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
   h->index_bufs.push_back(d);
@@ -1639,6 +1655,12 @@ int fdtd_release_memory(uint64_t keep_bytes) {
 const char* fdtd_version(void) { return "fdtd_b200 0.1.0 (sm_100a)"; }
 
 int fdtd_engine_create(const fdtd_grid_desc* desc, void* stream, fdtd_engine** out) {
+  return fdtd_engine_create_with(desc, stream, nullptr, nullptr, nullptr, out);
+}
+
+int fdtd_engine_create_with(const fdtd_grid_desc* desc, void* stream, fdtd_alloc_fn alloc, fdtd_free_fn release,
+                            void* user, fdtd_engine** out) {
+  if (!alloc != !release) return fail(FDTD_ERR_INVALID_ARG, "an allocator needs both functions");
   if (!desc || !out) return fail(FDTD_ERR_INVALID_ARG, "null descriptor or output pointer");
   *out = nullptr;
   if (desc->nx < 3 || desc->ny < 3 || desc->nz < 3)
@@ -1682,6 +1704,7 @@ int fdtd_engine_create(const fdtd_grid_desc* desc, void* stream, fdtd_engine** o
   for (int f = 0; f < 6; ++f)
     if (desc->boundary[f] == FDTD_BND_PMC) h->pmc = true;
   h->stream = static_cast<cudaStream_t>(stream);
+  h->mem = DeviceMemory{alloc, release, user};
   h->NX = desc->nx;
   h->NY = desc->ny;
   h->NZ = desc->nz;
@@ -1755,36 +1778,36 @@ int fdtd_engine_destroy(fdtd_engine* h) {
   // work on the engine's own streams reads the arrays too
   if (h->aux) cudaStreamSynchronize(h->aux);
   if (h->adj.rev) cudaStreamSynchronize(h->adj.rev);
-  for (float* p : h->owned) pool_free(p, h->stream);
+  for (float* p : h->owned) h->mem.free(p, h->stream);
   for (auto& pl : h->poles) {
-    pool_free(pl.drive, h->stream);
-    pool_free(pl.inv_eps, h->stream);
-    pool_free(pl.pol, h->stream);
-    pool_free(pl.cur, h->stream);
+    h->mem.free(pl.drive, h->stream);
+    h->mem.free(pl.inv_eps, h->stream);
+    h->mem.free(pl.pol, h->stream);
+    h->mem.free(pl.cur, h->stream);
   }
   for (auto& l : h->lines) {
-    pool_free(l.e_hist, h->stream);
-    pool_free(l.h_hist, h->stream);
+    h->mem.free(l.e_hist, h->stream);
+    h->mem.free(l.h_hist, h->stream);
   }
-  for (auto& ck : h->checkpoints) pool_free(ck.store, h->stream);
-  pool_free(h->d_terms, h->stream);
-  pool_free(h->d_poles, h->stream);
-  pool_free(h->d_regions, h->stream);
-  for (int* p : h->index_bufs) pool_free(p, h->stream);
-  pool_free(h->d_flush, h->stream);
-  pool_free(h->d_warp_class, h->stream);
-  pool_free(h->d_quad_class, h->stream);
-  for (float* p : h->adj.bufs) pool_free(p, h->stream);
-  pool_free(h->d_status, h->stream);
-  pool_free(h->d_base, h->stream);
-  pool_free(h->samples, h->stream);
-  pool_free(h->w_e, h->stream);
-  pool_free(h->w_h, h->stream);
-  pool_free(h->acc_re, h->stream);
-  pool_free(h->acc_im, h->stream);
-  pool_free(h->cmp_re, h->stream);
-  pool_free(h->cmp_im, h->stream);
-  pool_free(h->d_spectra, h->stream);
+  for (auto& ck : h->checkpoints) h->mem.free(ck.store, h->stream);
+  h->mem.free(h->d_terms, h->stream);
+  h->mem.free(h->d_poles, h->stream);
+  h->mem.free(h->d_regions, h->stream);
+  for (int* p : h->index_bufs) h->mem.free(p, h->stream);
+  h->mem.free(h->d_flush, h->stream);
+  h->mem.free(h->d_warp_class, h->stream);
+  h->mem.free(h->d_quad_class, h->stream);
+  for (float* p : h->adj.bufs) h->mem.free(p, h->stream);
+  h->mem.free(h->d_status, h->stream);
+  h->mem.free(h->d_base, h->stream);
+  h->mem.free(h->samples, h->stream);
+  h->mem.free(h->w_e, h->stream);
+  h->mem.free(h->w_h, h->stream);
+  h->mem.free(h->acc_re, h->stream);
+  h->mem.free(h->acc_im, h->stream);
+  h->mem.free(h->cmp_re, h->stream);
+  h->mem.free(h->cmp_im, h->stream);
+  h->mem.free(h->d_spectra, h->stream);
   for (cudaEvent_t e : {h->ev_fork, h->ev_join, h->ev_gat[0], h->ev_gat[1]})
     if (e) cudaEventDestroy(e);
   if (h->aux) cudaStreamDestroy(h->aux);
@@ -1793,6 +1816,7 @@ int fdtd_engine_destroy(fdtd_engine* h) {
   if (h->adj.rev) cudaStreamDestroy(h->adj.rev);
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);
+  if (!h->mem.caller_alloc) cudaStreamSynchronize(h->stream);  // the pool gives its memory back here
   delete h;
   return 0;
 }
@@ -1818,7 +1842,7 @@ int fdtd_engine_set_storage(fdtd_engine* h, int kind, const float* scales) {
         for (float** buf : {&h->E[b][c], &h->H[b][c]}) {
           auto it = std::find(h->owned.begin(), h->owned.end(), *buf);
           if (it != h->owned.end()) h->owned.erase(it);
-          pool_free(*buf, h->stream);
+          h->mem.free(*buf, h->stream);
           *buf = nullptr;
         }
     h->storage = kind;
@@ -2000,10 +2024,10 @@ int fdtd_engine_add_pole(fdtd_engine* h, int comp, int kind, const int* box, con
   ph.state_floats =
       static_cast<int64_t>((static_cast<size_t>(rows) * nkk * (h->storage == kStoreBF16 ? 2 : 4) + 3) / 4);
   const size_t sbytes = static_cast<size_t>(ph.state_floats) * sizeof(float);
-  CUDA_TRY(pool_alloc(&ph.drive, bytes, h->stream));
-  CUDA_TRY(pool_alloc(&ph.inv_eps, bytes, h->stream));
-  CUDA_TRY(pool_alloc(&ph.pol, sbytes, h->stream));
-  CUDA_TRY(pool_alloc(&ph.cur, sbytes, h->stream));
+  CUDA_TRY(h->mem.alloc(&ph.drive, bytes, h->stream));
+  CUDA_TRY(h->mem.alloc(&ph.inv_eps, bytes, h->stream));
+  CUDA_TRY(h->mem.alloc(&ph.pol, sbytes, h->stream));
+  CUDA_TRY(h->mem.alloc(&ph.cur, sbytes, h->stream));
   CUDA_TRY(cudaMemsetAsync(ph.drive, 0, bytes, h->stream));
   CUDA_TRY(cudaMemsetAsync(ph.inv_eps, 0, bytes, h->stream));
   CUDA_TRY(cudaMemsetAsync(ph.pol, 0, sbytes, h->stream));
@@ -2214,8 +2238,8 @@ int fdtd_engine_add_aux_line(fdtd_engine* h, int n_e, const float* e_decay, cons
   AuxLine l;
   l.ne = n_e;
   l.n_steps = n_steps;
-  CUDA_TRY(pool_alloc(&l.e_hist, sizeof(float) * static_cast<size_t>(n_steps) * n_e, h->stream));
-  CUDA_TRY(pool_alloc(&l.h_hist, sizeof(float) * static_cast<size_t>(n_steps) * n_e, h->stream));
+  CUDA_TRY(h->mem.alloc(&l.e_hist, sizeof(float) * static_cast<size_t>(n_steps) * n_e, h->stream));
+  CUDA_TRY(h->mem.alloc(&l.h_hist, sizeof(float) * static_cast<size_t>(n_steps) * n_e, h->stream));
   float *ed, *ecu, *hd, *hcu, *src, *e, *hh;
   int rc = dev_copy(h, &ed, e_decay, n_e);
   if (!rc) rc = dev_copy(h, &ecu, e_curl, n_e);
@@ -2263,7 +2287,7 @@ int fdtd_engine_add_line_patch(fdtd_engine* h, int comp, const int* box, const f
   for (int v : host_idx)
     if (v < 0 || v >= limit) return fail(FDTD_ERR_INVALID_ARG, "line patch sample index outside the incident line");
   int* idx = nullptr;
-  CUDA_TRY(pool_alloc(&idx, sizeof(int) * axis_len, h->stream));
+  CUDA_TRY(h->mem.alloc(&idx, sizeof(int) * axis_len, h->stream));
   CUDA_TRY(cudaMemcpyAsync(idx, host_idx.data(), sizeof(int) * axis_len, cudaMemcpyHostToDevice, h->stream));
   CUDA_TRY(cudaStreamSynchronize(h->stream));
   h->owned.push_back(reinterpret_cast<float*>(idx));
@@ -2306,22 +2330,22 @@ int set_dft_impl(fdtd_engine* h, int n_freq, const double* omega, int n_steps, c
     return fail(FDTD_ERR_INVALID_ARG, "bad DFT arguments");
   h->n_freq = n_freq;
   h->dft_steps = n_steps;
-  pool_free(h->w_e, h->stream);
-  pool_free(h->w_h, h->stream);
-  CUDA_TRY(pool_alloc(&h->w_e, sizeof(float2) * static_cast<size_t>(n_freq) * n_steps, h->stream));
-  CUDA_TRY(pool_alloc(&h->w_h, sizeof(float2) * static_cast<size_t>(n_freq) * n_steps, h->stream));
+  h->mem.free(h->w_e, h->stream);
+  h->mem.free(h->w_h, h->stream);
+  CUDA_TRY(h->mem.alloc(&h->w_e, sizeof(float2) * static_cast<size_t>(n_freq) * n_steps, h->stream));
+  CUDA_TRY(h->mem.alloc(&h->w_h, sizeof(float2) * static_cast<size_t>(n_freq) * n_steps, h->stream));
   const size_t n_window = static_cast<size_t>(n_steps) * (per_freq ? n_freq : 1);
   double *d_omega = nullptr, *d_window = nullptr;
-  CUDA_TRY(pool_alloc(&d_omega, sizeof(double) * n_freq, h->stream));
-  CUDA_TRY(pool_alloc(&d_window, sizeof(double) * n_window, h->stream));
+  CUDA_TRY(h->mem.alloc(&d_omega, sizeof(double) * n_freq, h->stream));
+  CUDA_TRY(h->mem.alloc(&d_window, sizeof(double) * n_window, h->stream));
   CUDA_TRY(cudaMemcpyAsync(d_omega, omega, sizeof(double) * n_freq, cudaMemcpyHostToDevice, h->stream));
   CUDA_TRY(cudaMemcpyAsync(d_window, window, sizeof(double) * n_window, cudaMemcpyHostToDevice, h->stream));
   dft_weight_kernel<<<256, 256, 0, h->stream>>>(n_freq, n_steps, d_omega, d_window, per_freq, h->desc.dt, h->w_e,
                                                 h->w_h);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaStreamSynchronize(h->stream));
-  pool_free(d_omega, h->stream);
-  pool_free(d_window, h->stream);
+  h->mem.free(d_omega, h->stream);
+  h->mem.free(d_window, h->stream);
   return 0;
 }
 
@@ -2444,7 +2468,7 @@ int fdtd_engine_finalize(fdtd_engine* h) {
         return fail(FDTD_ERR_UNSUPPORTED, "nonlinear media with poles run launch variants 1-3, 10 and 11");
     }
     const int64_t n = static_cast<int64_t>(h->nl_cells_h.size() / 4);
-    CUDA_TRY(pool_alloc(&h->d_nl_cells, sizeof(int4) * n, h->stream));
+    CUDA_TRY(h->mem.alloc(&h->d_nl_cells, sizeof(int4) * n, h->stream));
     h->owned.push_back(reinterpret_cast<float*>(h->d_nl_cells));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     CUDA_TRY(cudaMemcpy(h->d_nl_cells, h->nl_cells_h.data(), sizeof(int4) * n, cudaMemcpyHostToDevice));
@@ -2622,13 +2646,13 @@ int fdtd_engine_finalize(fdtd_engine* h) {
   if (rc) return rc;
   h->n_flush = static_cast<int>(fl.size());
   if (h->n_samples > 0) {
-    CUDA_TRY(pool_alloc(&h->samples, sizeof(float) * static_cast<size_t>(h->M) * h->n_samples, h->stream));
+    CUDA_TRY(h->mem.alloc(&h->samples, sizeof(float) * static_cast<size_t>(h->M) * h->n_samples, h->stream));
     if (h->n_freq > 0) {
       const size_t acc = static_cast<size_t>(h->n_freq) * h->n_samples;
-      CUDA_TRY(pool_alloc(&h->acc_re, sizeof(float) * acc, h->stream));
-      CUDA_TRY(pool_alloc(&h->acc_im, sizeof(float) * acc, h->stream));
-      CUDA_TRY(pool_alloc(&h->cmp_re, sizeof(float) * acc, h->stream));
-      CUDA_TRY(pool_alloc(&h->cmp_im, sizeof(float) * acc, h->stream));
+      CUDA_TRY(h->mem.alloc(&h->acc_re, sizeof(float) * acc, h->stream));
+      CUDA_TRY(h->mem.alloc(&h->acc_im, sizeof(float) * acc, h->stream));
+      CUDA_TRY(h->mem.alloc(&h->cmp_re, sizeof(float) * acc, h->stream));
+      CUDA_TRY(h->mem.alloc(&h->cmp_im, sizeof(float) * acc, h->stream));
       CUDA_TRY(cudaMemsetAsync(h->acc_re, 0, sizeof(float) * acc, h->stream));
       CUDA_TRY(cudaMemsetAsync(h->acc_im, 0, sizeof(float) * acc, h->stream));
       CUDA_TRY(cudaMemsetAsync(h->cmp_re, 0, sizeof(float) * acc, h->stream));
@@ -2650,11 +2674,11 @@ int fdtd_engine_finalize(fdtd_engine* h) {
   }
   {
     const int64_t kblocks = (h->NZ + kWarpOut - 1) / kWarpOut;
-    CUDA_TRY(pool_alloc(&h->d_warp_class, static_cast<size_t>(h->NX) * kblocks * h->NY, h->stream));
+    CUDA_TRY(h->mem.alloc(&h->d_warp_class, static_cast<size_t>(h->NX) * kblocks * h->NY, h->stream));
     h->class_key = 0;
     h->quad_key = 0;
     if (h->storage == kStoreF32 && has_coef(h))
-      CUDA_TRY(pool_alloc(&h->d_quad_class, static_cast<size_t>(h->NX) * h->NY * (h->P / 4), h->stream));
+      CUDA_TRY(h->mem.alloc(&h->d_quad_class, static_cast<size_t>(h->NX) * h->NY * (h->P / 4), h->stream));
     if (h->storage == kStoreF32) {
       rc = dev_alloc(h, &h->d_ztab_h, 4 * static_cast<size_t>(h->P));
       if (!rc) rc = dev_alloc(h, &h->d_ztab_e, 4 * static_cast<size_t>(h->P));
@@ -2668,9 +2692,9 @@ int fdtd_engine_finalize(fdtd_engine* h) {
       err = prepare_quad_step(h->cpml, has_coef(h), h->uniform_grid);
       if (err != 0) return cuda_fail(static_cast<cudaError_t>(err), "shared memory of quad_step_kernel");
     }
-    CUDA_TRY(pool_alloc(&h->d_status, sizeof(int), h->stream));
+    CUDA_TRY(h->mem.alloc(&h->d_status, sizeof(int), h->stream));
     CUDA_TRY(cudaMemsetAsync(h->d_status, 0, sizeof(int), h->stream));
-    CUDA_TRY(pool_alloc(&h->d_base, sizeof(int), h->stream));
+    CUDA_TRY(h->mem.alloc(&h->d_base, sizeof(int), h->stream));
     CUDA_TRY(cudaMemsetAsync(h->d_base, 0, sizeof(int), h->stream));
   }
   {
@@ -2882,11 +2906,11 @@ static void state_buffers(fdtd_engine* h, std::vector<std::pair<float*, size_t>>
 
 static int checkpoint_alloc(fdtd_engine* h, Checkpoint& ck, const std::vector<std::pair<float*, size_t>>& bufs) {
   if (ck.store && ck.bufs.size() == bufs.size()) return 0;
-  pool_free(ck.store, h->stream);
+  h->mem.free(ck.store, h->stream);
   ck.store = nullptr;
   size_t total = 0;
   for (const auto& b : bufs) total += (b.second + 63) / 64 * 64;  // 256-byte aligned views
-  CUDA_TRY(pool_alloc(&ck.store, std::max<size_t>(total, 1) * sizeof(float), h->stream));
+  CUDA_TRY(h->mem.alloc(&ck.store, std::max<size_t>(total, 1) * sizeof(float), h->stream));
   ck.bufs.clear();
   size_t off = 0;
   for (const auto& b : bufs) {
@@ -3005,7 +3029,7 @@ int fdtd_engine_autotune(fdtd_engine* h, int* tile_rows, int* chunk_planes) {
   h->TY = best_ty;
   rc = fdtd_engine_checkpoint_load(h, slot);
   if (rc) return rc;
-  pool_free(h->checkpoints[slot].store, h->stream);
+  h->mem.free(h->checkpoints[slot].store, h->stream);
   h->checkpoints.pop_back();
   h->pending = 0;
   h->pending_base = next_step;
@@ -3139,7 +3163,7 @@ int fdtd_engine_set_prefetch(fdtd_engine* h, int planes) {
 static int adj_alloc(fdtd_engine* h, float** out, size_t n) {
   *out = nullptr;
   if (n == 0) return 0;
-  CUDA_TRY(pool_alloc(out, n * sizeof(float), h->stream));
+  CUDA_TRY(h->mem.alloc(out, n * sizeof(float), h->stream));
   CUDA_TRY(cudaMemsetAsync(*out, 0, n * sizeof(float), h->stream));
   h->adj.bufs.push_back(*out);
   return 0;
@@ -3178,9 +3202,9 @@ int fdtd_engine_adjoint_init(fdtd_engine* h, const int* design_boxes, int max_se
     }
     float** dgp = nullptr;
     float** dgc = nullptr;
-    CUDA_TRY(pool_alloc(&dgp, sizeof(float*) * gp.size(), h->stream));
+    CUDA_TRY(h->mem.alloc(&dgp, sizeof(float*) * gp.size(), h->stream));
     a.bufs.push_back(reinterpret_cast<float*>(dgp));
-    CUDA_TRY(pool_alloc(&dgc, sizeof(float*) * gc.size(), h->stream));
+    CUDA_TRY(h->mem.alloc(&dgc, sizeof(float*) * gc.size(), h->stream));
     a.bufs.push_back(reinterpret_cast<float*>(dgc));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     CUDA_TRY(cudaMemcpy(dgp, gp.data(), sizeof(float*) * gp.size(), cudaMemcpyHostToDevice));
@@ -3568,6 +3592,7 @@ struct fdtd_batch {
   // which capture is not permitted
   cudaStream_t cap = nullptr;
   int** d_bases = nullptr;
+  DeviceMemory mem;  // the first engine's
   cudaGraphExec_t exec = nullptr;
   int M = 0;
   float last_ms = 0.0f;
@@ -3652,6 +3677,7 @@ int fdtd_batch_create(fdtd_engine* const* engines, int n, void* stream, fdtd_bat
   fdtd_batch* b = new fdtd_batch();
   b->eng.assign(engines, engines + n);
   b->stream = st;
+  b->mem = engines[0]->mem;
   b->M = M;
   b->streams.resize(n, nullptr);
   b->join.resize(n, nullptr);
@@ -3663,7 +3689,7 @@ int fdtd_batch_create(fdtd_engine* const* engines, int n, void* stream, fdtd_bat
     err = cudaStreamCreateWithFlags(&b->streams[i], cudaStreamNonBlocking);
     if (err == cudaSuccess) err = cudaEventCreateWithFlags(&b->join[i], cudaEventDisableTiming);
   }
-  if (err == cudaSuccess) err = pool_alloc(&b->d_bases, sizeof(int*) * n, b->stream);
+  if (err == cudaSuccess) err = b->mem.alloc(&b->d_bases, sizeof(int*) * n, b->stream);
   if (err == cudaSuccess) {
     std::vector<int*> bases(n);
     for (int i = 0; i < n; ++i) bases[i] = engines[i]->d_base;
@@ -3691,7 +3717,7 @@ int fdtd_batch_destroy(fdtd_batch* b) {
   if (b->fork) cudaEventDestroy(b->fork);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
-  pool_free(b->d_bases, b->stream);
+  b->mem.free(b->d_bases, b->stream);
   delete b;
   return 0;
 }

@@ -52,11 +52,28 @@ def pin_scene(cs):
     )
 
 
+@_lib.ALLOC_FN
+def _torch_alloc(nbytes, device, stream, user):
+    try:
+        return torch.cuda.caching_allocator_alloc(nbytes, device, stream or 0)
+    except Exception:  # out of memory: the engine reports it
+        return None
+
+
+@_lib.FREE_FN
+def _torch_free(memory, user):
+    torch.cuda.caching_allocator_delete(memory)
+
+
 def release_memory(keep_bytes: int = 0, device=None) -> None:
-    """Give the device memory that closed solvers left in the library's pool (at most
-    4 GiB) back to the device, but for ``keep_bytes``."""
+    """Give the device memory that closed solvers left back to the device.  It lies in
+    torch's caching allocator, beside that of freed tensors, and serves whatever torch
+    allocates next, so this is needed for other users of the device only.
+    ``keep_bytes`` is how much of the library's own pool may stay; the solvers of this
+    module do not use that pool."""
     with torch.cuda.device(torch.device("cuda") if device is None else torch.device(device)):
         _lib.check(_lib.load().fdtd_release_memory(int(keep_bytes)), "release_memory")
+        torch.cuda.empty_cache()
 
 
 class B200FDTD:
@@ -141,8 +158,9 @@ class B200FDTD:
             desc.tile_rows = self.tile_rows
             desc.chunk_planes = self.chunk_planes
             handle = ctypes.c_void_p()
-            _lib.check(lib.fdtd_engine_create(ctypes.byref(desc), ctypes.c_void_p(stream.cuda_stream), ctypes.byref(handle)),
-                       "fdtd_engine_create")
+            _lib.check(lib.fdtd_engine_create_with(ctypes.byref(desc), ctypes.c_void_p(stream.cuda_stream), _torch_alloc,
+                                                   _torch_free, None, ctypes.byref(handle)),
+                       "fdtd_engine_create_with")
             h = handle
             if self.storage != "fp32" or self.storage_scales_arg is not None:
                 sc = None
