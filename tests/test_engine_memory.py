@@ -13,6 +13,7 @@ from conftest import load_package
 
 pytestmark = pytest.mark.gpu
 MIB = 1 << 20
+FIELDS = ("Ex", "Ey", "Ez", "Hx", "Hy", "Hz")
 
 
 def _compiled(wm, n=160):
@@ -44,6 +45,62 @@ def test_a_closed_solvers_memory_serves_the_next_tensors():
     del tensors
     torch.cuda.empty_cache()
     assert _free() >= before - 4 * MIB
+
+
+def _tfsf(wm, boundary):
+    sc = wm.Scene(cells=(32, 28, 30), spacing=25e-9, pml_cells=6, boundary=boundary)
+    sc.structures.append(wm.Structure(wm.Box((12, 11, 12), (18, 16, 17)), wm.Medium(eps_r=3.0)))
+    sc.structures.append(wm.Structure(wm.Sphere((16.0, 14.0, 15.0), 3.0), wm.Medium.lorentz(2.0, 3.0, 250e12, 20e12)))
+    pulse = wm.GaussianPulse(300e12, 100e12, delay=0.5e-15)
+    if 2 in boundary or 3 in boundary:
+        sc.sources.append(wm.PointDipole((14, 13, 14), "Ex", pulse, width=25e-9))
+        if 3 in boundary:
+            sc.bloch_k = (2e6, 1e6, 0.0)
+    else:
+        sc.sources.append(wm.PlaneWaveTFSF((1, 0, 0), (0, 0, 1), pulse, (9, 9, 9), (23, 19, 21)))
+    sc.monitors.append(wm.PlaneMonitor("plane", 2, 15, frequencies=(250e12, 300e12)))
+    return sc
+
+
+@pytest.mark.parametrize("storage,boundary", [
+    ("fp32", (1,) * 6), ("fp16", (1,) * 6), ("bf16", (1,) * 6), ("fp32", (4,) * 6), ("fp16", (4,) * 6),
+    ("fp32", (2, 2, 2, 2, 1, 1)), ("fp32", (3, 3, 3, 3, 1, 1)),
+])
+def test_an_engine_reads_nothing_that_its_memory_held_before(storage, boundary, monkeypatch):
+    """The same scales, fields and spectra on memory that holds 1.2e30 everywhere."""
+    wm = load_package()
+    held = {}
+
+    @wm._lib.ALLOC_FN
+    def alloc(nbytes, device, stream, user):
+        t = torch.full((nbytes,), 0x71, dtype=torch.uint8, device="cuda")
+        held[t.data_ptr()] = t
+        return t.data_ptr()
+
+    @wm._lib.FREE_FN
+    def release(memory, user):
+        del held[memory]
+
+    cs = wm.compile_scene(_tfsf(wm, boundary), 40)
+    runs = []
+    for poisoned in (False, True):
+        if poisoned:
+            monkeypatch.setattr(wm.solver, "_torch_alloc", alloc)
+            monkeypatch.setattr(wm.solver, "_torch_free", release)
+        solver = wm.solver.B200FDTD(cs, storage=storage).init_field()
+        assert bool(held) == poisoned
+        scales = solver.storage_scales()
+        solver.step_range(0, 40)
+        fields = {n: solver.field(n) for n in FIELDS}
+        spectra = {c: v.clone() for c, v in solver.monitor_results()["plane"].items()}
+        solver.close()
+        runs.append((scales, fields, spectra))
+    assert not held
+    assert runs[0][0] == runs[1][0]
+    for k in (1, 2):
+        for name, v in runs[0][k].items():
+            assert torch.equal(v, runs[1][k][name]), name
+    assert float(runs[0][1]["Ez"].abs().max()) > 0
 
 
 def test_an_engine_without_an_allocator_gives_its_memory_back_at_once():

@@ -2238,8 +2238,11 @@ int fdtd_engine_add_aux_line(fdtd_engine* h, int n_e, const float* e_decay, cons
   AuxLine l;
   l.ne = n_e;
   l.n_steps = n_steps;
-  CUDA_TRY(h->mem.alloc(&l.e_hist, sizeof(float) * static_cast<size_t>(n_steps) * n_e, h->stream));
-  CUDA_TRY(h->mem.alloc(&l.h_hist, sizeof(float) * static_cast<size_t>(n_steps) * n_e, h->stream));
+  const size_t hist_bytes = sizeof(float) * static_cast<size_t>(n_steps) * n_e;
+  CUDA_TRY(h->mem.alloc(&l.e_hist, hist_bytes, h->stream));
+  CUDA_TRY(h->mem.alloc(&l.h_hist, hist_bytes, h->stream));
+  // a row of H holds n_e - 1 values; the scale estimate of FP16 storage reads it whole
+  CUDA_TRY(cudaMemsetAsync(l.h_hist, 0, hist_bytes, h->stream));
   float *ed, *ecu, *hd, *hcu, *src, *e, *hh;
   int rc = dev_copy(h, &ed, e_decay, n_e);
   if (!rc) rc = dev_copy(h, &ecu, e_curl, n_e);
