@@ -5,11 +5,13 @@ from __future__ import annotations
 
 import ctypes
 import gc
+import subprocess
+import sys
 
 import pytest
 import torch
 
-from conftest import load_package
+from conftest import ROOT, load_package
 
 pytestmark = pytest.mark.gpu
 MIB = 1 << 20
@@ -101,6 +103,29 @@ def test_an_engine_reads_nothing_that_its_memory_held_before(storage, boundary, 
         for name, v in runs[0][k].items():
             assert torch.equal(v, runs[1][k][name]), name
     assert float(runs[0][1]["Ez"].abs().max()) > 0
+
+
+@pytest.mark.parametrize("held", ["solver", "batch", "everything"])
+def test_solvers_may_be_open_when_the_interpreter_ends(held):
+    """Nothing is closed: the engines go with the modules whose functions free them."""
+    code = f"""
+import sys
+sys.path.insert(0, {str(ROOT / "tests")!r})
+from conftest import ROOT, load_package
+wm = load_package()
+cs = wm.compile_scene(wm.Scene(cells=(20, 20, 20), spacing=25e-9, pml_cells=4), 64)
+solver = wm.solver.B200FDTD(cs).init_field()
+solver.step_range(0, 4)
+if {held!r} != "solver":
+    batch = wm.solver.B200Batch([wm.solver.B200FDTD(cs) for _ in range(2)])
+    batch.step_range(0, 40)
+if {held!r} == "everything":
+    sys.keep = [solver, batch]  # beyond the modules
+    sys.keep.append(sys.keep)
+print("stepped")
+"""
+    done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0 and done.stdout.split() == ["stepped"], (done.returncode, done.stderr[-2000:])
 
 
 def test_an_engine_without_an_allocator_gives_its_memory_back_at_once():

@@ -52,17 +52,23 @@ def pin_scene(cs):
     )
 
 
+# Called back by the library (fdtd_engine_create_with).  A solver holds the two objects
+# for as long as its engine lives, which at the end of the interpreter can be longer
+# than this module's names; what they call is bound here for the same reason.
 @_lib.ALLOC_FN
-def _torch_alloc(nbytes, device, stream, user):
+def _torch_alloc(nbytes, device, stream, user, alloc=torch.cuda.caching_allocator_alloc):
     try:
-        return torch.cuda.caching_allocator_alloc(nbytes, device, stream or 0)
+        return alloc(nbytes, device, stream or 0)
     except Exception:  # out of memory: the engine reports it
         return None
 
 
 @_lib.FREE_FN
-def _torch_free(memory, user):
-    torch.cuda.caching_allocator_delete(memory)
+def _torch_free(memory, user, delete=torch.cuda.caching_allocator_delete):
+    try:
+        delete(memory)
+    except Exception:  # torch is being unloaded with the process
+        pass
 
 
 def release_memory(keep_bytes: int = 0, device=None) -> None:
@@ -107,6 +113,7 @@ class B200FDTD:
         self.pole_ids: list[int] = []
         self.steps_done = 0
         self._spectra = None  # layout of monitor_results
+        self._memory = (_torch_alloc, _torch_free)  # the engines' device memory
         self._keep: list = []
 
     # ------------------------------------------------------------------ setup
@@ -158,8 +165,8 @@ class B200FDTD:
             desc.tile_rows = self.tile_rows
             desc.chunk_planes = self.chunk_planes
             handle = ctypes.c_void_p()
-            _lib.check(lib.fdtd_engine_create_with(ctypes.byref(desc), ctypes.c_void_p(stream.cuda_stream), _torch_alloc,
-                                                   _torch_free, None, ctypes.byref(handle)),
+            _lib.check(lib.fdtd_engine_create_with(ctypes.byref(desc), ctypes.c_void_p(stream.cuda_stream), *self._memory,
+                                                   None, ctypes.byref(handle)),
                        "fdtd_engine_create_with")
             h = handle
             if self.storage != "fp32" or self.storage_scales_arg is not None:
