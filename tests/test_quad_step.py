@@ -125,6 +125,26 @@ def test_many_terms_on_a_row_shorten_the_chunks():
         np.testing.assert_array_equal(fields[1][n], fields[2][n])
 
 
+def test_poles_in_the_step_kernel_run_the_warp_kernels_launch():
+    """Without the ADE pass the warp kernel runs, on its own chunks; with it again, the
+    quad tile as before.  A launch that was set stays."""
+    wm = load_package()
+    cs = _scene(wm, (60, 50, 40), 4, (1,) * 6)
+    solver = wm.solver.B200FDTD(cs).init_field()
+    first = solver.get_launch()
+    solver.set_ade_pass(False)
+    off = solver.get_launch()
+    solver.step_range(0, 4)
+    solver.set_ade_pass(True)
+    assert solver.get_launch() == first
+    solver.set_launch(2, 0, 0)
+    assert off == (11,) + solver.get_launch()[1:]
+    solver.set_launch(11, 3, 7)
+    solver.set_ade_pass(False)
+    assert solver.get_launch() == (11, 3, 7)
+    solver.close()
+
+
 def test_rows_beyond_a_tile_run_another_kernel():
     wm = load_package()
     solver = wm.solver.B200FDTD(_scene(wm, (8, 8, 512), 2, (1,) * 6)).init_field()

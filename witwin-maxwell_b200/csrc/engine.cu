@@ -786,7 +786,7 @@ struct fdtd_engine {
   // exchange, tile_kernel.cu); 11 = quad-tile kernel (four z cells per thread,
   // bulk-copied planes, quad_kernel.cu).
   int variant = kDefaultVariant;
-  bool launch_set = false;  // by fdtd_engine_set_launch
+  bool launch_set = false;  // by fdtd_engine_set_launch or autotune
   int pf_dist = kDefaultPrefetch;
   int cur = 0;  // index of the buffer holding the current state
   float* E[2][3] = {};
@@ -1153,7 +1153,8 @@ void default_quad(fdtd_engine* h, int ty, int cx) {
 }
 
 void default_tiles(fdtd_engine* h) {
-  if (h->variant == kQuadVariant) {
+  // with poles in the step kernel the warp kernel runs in the quad-tile kernel's place
+  if (h->variant == kQuadVariant && (h->ade_pass || h->poles.empty())) {
     default_quad(h, h->desc.tile_rows, h->desc.chunk_planes);
     if (h->quad.threads > 0) return;
     default_quad(h, 0, h->desc.chunk_planes);  // the caller's tile rows do not fit
@@ -3026,6 +3027,7 @@ int fdtd_engine_autotune(fdtd_engine* h, int* tile_rows, int* chunk_planes) {
       }
     }
   }
+  h->launch_set = true;
   h->variant = best_var;
   if (best_var == kQuadVariant) default_quad(h, best_ty, best_cx);
   h->CX = best_cx;
@@ -3104,6 +3106,7 @@ int fdtd_engine_set_ade_pass(fdtd_engine* h, int on) {
   if (!on && h->nl_general >= 0 && !h->poles.empty())
     return fail(FDTD_ERR_UNSUPPORTED, "nonlinear media with poles need the ADE pass");
   h->ade_pass = on != 0;
+  if (h->variant == kQuadVariant && !h->launch_set) default_tiles(h);
   return 0;
 }
 
