@@ -176,6 +176,13 @@ __device__ __forceinline__ void ztab(float (&b)[4], float (&c)[4], float (&ik)[4
 
 // Injection terms `bits` of one phase (component base..base + 2) in plane i on
 // the quad at (j, k).
+// kTogether: a quad's loads go out together.  One after the other, their latencies make
+// a plane with many terms slow (24 dipoles over the same cells of a closed 128^3 box:
+// 224 us a step, 182 together; one in 182 x 212 x 158: 62.9 and 59.5).  In the kernels
+// with slab code the longer loop costs more than it gives on the thin terms of a TFSF
+// box, one cell of a quad each (one channel of the 257 x 257 x 193 grating, z slabs:
+// 308 us a step, 315 together).
+template <bool kTogether>
 __device__ __forceinline__ void quad_terms(const QuadTerms& terms, unsigned bits, int base, int n, int i, int j, int k,
                                            float (&v0)[4], float (&v1)[4], float (&v2)[4]) {
   for (; bits; bits &= bits - 1) {
@@ -185,31 +192,44 @@ __device__ __forceinline__ void quad_terms(const QuadTerms& terms, unsigned bits
     const float* row = t.coeff + (static_cast<int64_t>(li) * (t.j1 - t.j0) + lj) * (t.k1 - t.k0) - t.k0;
     const bool along_z = t.signal == nullptr && t.sample_axis == 2;
     const float* hist = t.aux_hist + static_cast<int64_t>(n) * t.aux_len;
-    // the quad's loads go out together: one after the other, their latencies make a
-    // plane with many terms slow (24 dipoles over the same cells of a closed 128^3
-    // box: 224 us a step, 182 together)
-    bool in[4];
-    float w[4], s[4];
-    const float one = t.signal != nullptr ? __ldg(t.signal + n)
-                      : along_z           ? 0.f
-                                          : __ldg(hist + __ldg(t.sample_index + (t.sample_axis == 0 ? li : lj)));
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      in[q] = k + q >= t.k0 && k + q < t.k1;
-      w[q] = in[q] ? __ldg(row + k + q) : 0.f;
-      s[q] = one;
-    }
-    if (along_z) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) s[q] = in[q] ? __ldg(hist + __ldg(t.sample_index + k + q - t.k0)) : 0.f;
-    }
     const int c = t.comp - base;
+    if constexpr (kTogether) {
+      bool in[4];
+      float w[4], s[4];
+      const float one = t.signal != nullptr ? __ldg(t.signal + n)
+                        : along_z           ? 0.f
+                                            : __ldg(hist + __ldg(t.sample_index + (t.sample_axis == 0 ? li : lj)));
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        in[q] = k + q >= t.k0 && k + q < t.k1;
+        w[q] = in[q] ? __ldg(row + k + q) : 0.f;
+        s[q] = one;
+      }
+      if (along_z) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s[q] = in[q] ? __ldg(hist + __ldg(t.sample_index + k + q - t.k0)) : 0.f;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float val = __fmul_rn(w[q], s[q]);
+        if (c == 0) v0[q] = in[q] ? __fmaf_rn(val, t.scale, v0[q]) : v0[q];
+        else if (c == 1) v1[q] = in[q] ? __fmaf_rn(val, t.scale, v1[q]) : v1[q];
+        else v2[q] = in[q] ? __fmaf_rn(val, t.scale, v2[q]) : v2[q];
+      }
+      continue;
+    }
+    float s = 0.f;
+    if (t.signal != nullptr) s = __ldg(t.signal + n);
+    else if (!along_z) s = __ldg(hist + __ldg(t.sample_index + (t.sample_axis == 0 ? li : lj)));
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const float val = __fmul_rn(w[q], s[q]);
-      if (c == 0) v0[q] = in[q] ? __fmaf_rn(val, t.scale, v0[q]) : v0[q];
-      else if (c == 1) v1[q] = in[q] ? __fmaf_rn(val, t.scale, v1[q]) : v1[q];
-      else v2[q] = in[q] ? __fmaf_rn(val, t.scale, v2[q]) : v2[q];
+      const int kk = k + q;
+      if (kk < t.k0 || kk >= t.k1) continue;
+      if (along_z) s = __ldg(hist + __ldg(t.sample_index + kk - t.k0));
+      const float val = __fmul_rn(__ldg(row + kk), s);
+      if (c == 0) v0[q] = __fmaf_rn(val, t.scale, v0[q]);
+      else if (c == 1) v1[q] = __fmaf_rn(val, t.scale, v1[q]);
+      else v2[q] = __fmaf_rn(val, t.scale, v2[q]);
     }
   }
 }
@@ -480,7 +500,7 @@ __device__ __forceinline__ void quad_march(const StepParams& p, const QuadTerms&
         fill4(hy, 0.f);
         fill4(hz, 0.f);
       }
-      if (tmask & terms.h_bits) quad_terms(terms, tmask & terms.h_bits, 3, n, i, j, k, hx, hy, hz);
+      if (tmask & terms.h_bits) quad_terms<kFold>(terms, tmask & terms.h_bits, 3, n, i, j, k, hx, hy, hz);
       // One writer for each quad of the ring: a thread that repeats the last item
       // reads the same H^{n-1/2} and, writing too, could be read by the item's own
       // thread before that has loaded it (the lanes of a warp need not run together).
@@ -597,7 +617,7 @@ __device__ __forceinline__ void quad_march(const StepParams& p, const QuadTerms&
           }
       }
       if (tmask & ~terms.h_bits) {
-        quad_terms(terms, tmask & ~terms.h_bits, 0, n, i, j, k, v0, v1, v2);
+        quad_terms<kFold>(terms, tmask & ~terms.h_bits, 0, n, i, j, k, v0, v1, v2);
         // scenes without TFSF end the E update on PEC faces (stepping.py:2316-2318)
         if (p.pec_clamp) {
           const bool zp0 = zf.first && p.bnd[4] == BND_PEC, zp1 = p.bnd[5] == BND_PEC;
