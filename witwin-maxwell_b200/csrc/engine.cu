@@ -1245,8 +1245,9 @@ int ensure_classified(fdtd_engine* h, const StepParams& p) {
   return 0;
 }
 
-// The poles run in the ADE pass after the step kernel (instead of inside it)
-// on FP32 storage with the scalar step kernels and no wrapped face.
+// The poles run in the ADE pass after the step kernel (instead of inside it) on FP32
+// storage: with the quad-tile kernel, and without wrapped faces with the scalar and
+// row-tile kernels.
 bool ade_pass_active(const fdtd_engine* h) {
   return h->ade_pass && h->n_ade_tiles > 0 && h->poles.size() <= static_cast<size_t>(kAdeMaxPoles) &&
          h->storage == kStoreF32 &&
@@ -1356,9 +1357,9 @@ int launch_aniso(fdtd_engine* h, const StepParams& p) {
   return 0;
 }
 
-// region: node box (x0, x1, y0, y1, z0, z1) to which the warp kernel's task
-// grid is restricted (a sub-grid of whole row blocks, z blocks and chunks that
-// covers it), or nullptr for the full step.  Only the scalar warp kernels take
+// region: node box (x0, x1, y0, y1, z0, z1) to which the task grid of the warp kernel
+// (whole row blocks, z blocks and chunks that cover it) or of the quad-tile kernel
+// (whole rows and chunks) is restricted, or nullptr for the full step.  Only these take
 // a region (region_ok); cells outside it keep stale values.
 int launch_step(fdtd_engine* h, int n, int slot, const int* region = nullptr) {
   if (!h->shifted.empty()) {

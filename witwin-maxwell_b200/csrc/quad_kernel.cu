@@ -26,8 +26,13 @@
 // that code (717 -> 560 warp instructions per plane with a 10-cell CPML, 130 ->
 // 122 us at 193 x 193 x 161; z-slab psi from the ring instead of from L2: -> 108 us).
 //
-// What bounds it: HBM.  See default_quad (engine.cu) for the tile rule and the
-// measured times.
+// What bounds it: without slab code the copies on large grids (257^3, one source: 0.89
+// of the measured copy rate; 182 x 212 x 158, less than one round of CTAs: 0.68).
+// With it the plane barrier, at which a warp in a slab holds its CTA, 19 warps and
+// one CTA per SM (193 x 193 x 161, 10 cells: DRAM at 0.46 of the copy rate, an issue in
+// 0.41 of the cycles, the barrier the largest stall).  On small grids the launch and the
+// latency of two planes (25 x 21 x 19: 14 us).  See default_quad (engine.cu) for the
+// tile rule and the measured times.
 //
 // Every mbarrier wait is bounded (StepParams::wait_limit polls).  A wait that
 // runs out records FDTD_ERR_TIMEOUT in p.status; the thread carries on without
