@@ -294,8 +294,8 @@ def run_reference_arm(args, wm, world, rank):
 # same kernels and grid; null otherwise.
 NCU_TRAFFIC = {
     "cells": 256 ** 3,
-    "kernels": {"warp_step_kernel<1,1,1,4,0>": 1055.3e6, "ade_pass_kernel": 372.1e6},
-    "launch": {"variant": 2, "chunk_planes": 13},
+    "kernels": {"quad_step_kernel<1,1,1>": 1003.1e6, "ade_pass_kernel": 379.5e6},
+    "launch": {"variant": 11, "chunk_planes": 10},
 }
 
 

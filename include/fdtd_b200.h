@@ -257,8 +257,10 @@ int fdtd_engine_checkpoint_save(fdtd_engine* h, int slot);
 int fdtd_engine_checkpoint_reserve(fdtd_engine* h, int n_slots);
 int fdtd_engine_checkpoint_load(fdtd_engine* h, int slot);
 
-/* Tile shape selection: time the candidate (tile_rows, chunk_planes) pairs on
- * the bound scene (state is saved and restored) and keep the fastest. */
+/* Launch selection: time the present launch and the candidates (chunk lengths; every
+ * variant that the engine takes, but on an engine that runs variant 11 its tiles only)
+ * on the bound scene (state is saved and restored) and keep the fastest, the present
+ * one unless another is 2 % faster. */
 int fdtd_engine_autotune(fdtd_engine* h, int* tile_rows, int* chunk_planes);
 /* Launch configuration of the fused step kernel.  Variants 1-3: the scalar
  * warp kernel (one z cell per lane) with a register budget of about 100 (1),
@@ -277,7 +279,7 @@ int fdtd_engine_autotune(fdtd_engine* h, int* tile_rows, int* chunk_planes);
  * or PMC faces, 2 otherwise; reduced storage runs 2 only.
  * chunk_planes is the number of x planes each warp marches through (0 picks
  * the variant's default).  tile_rows is the number of rows of a CTA of variant 11
- * (0 picks its default; FDTD_ERR_INVALID_ARG when a CTA cannot hold them); the
+ * (0 picks its default, which at finalize counts the injection terms; FDTD_ERR_INVALID_ARG when a CTA cannot hold them); the
  * other variants ignore it.  Autotuning an engine that runs 11 picks its tile. */
 int fdtd_engine_set_launch(fdtd_engine* h, int variant, int tile_rows, int chunk_planes);
 int fdtd_engine_get_launch(fdtd_engine* h, int* variant, int* tile_rows, int* chunk_planes);
@@ -326,8 +328,9 @@ int fdtd_engine_last_ms(fdtd_engine* h, float* ms);
 typedef struct fdtd_batch fdtd_batch;
 int fdtd_batch_create(fdtd_engine* const* engines, int n, void* stream, fdtd_batch** out);
 int fdtd_batch_destroy(fdtd_batch* b);
-/* Launch-shape autotune per size class (node counts rounded to 32): the first
- * engine of each class runs fdtd_engine_autotune, the others take its pick. */
+/* Launch-shape autotune per class (node counts rounded to 32, CPML, faces, storage,
+ * kernel): the first engine of each class runs fdtd_engine_autotune, the others take
+ * its pick, or run it themselves where they cannot. */
 int fdtd_batch_autotune(fdtd_batch* b);
 int fdtd_batch_step_range(fdtd_batch* b, int n0, int n1);
 int fdtd_batch_last_ms(fdtd_batch* b, float* ms);
