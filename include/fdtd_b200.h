@@ -278,9 +278,10 @@ int fdtd_engine_autotune(fdtd_engine* h, int* tile_rows, int* chunk_planes);
  * 10).  Default: 11 for FP32 engines it takes; else 10 without CPML, periodic, Bloch
  * or PMC faces, 2 otherwise; reduced storage runs 2 only.
  * chunk_planes is the number of x planes each warp marches through (0 picks
- * the variant's default).  tile_rows is the number of rows of a CTA of variant 11
- * (0 picks its default, which at finalize counts the injection terms; FDTD_ERR_INVALID_ARG when a CTA cannot hold them); the
- * other variants ignore it.  Autotuning an engine that runs 11 picks its tile. */
+ * the variant's default).  tile_rows is the number of rows of a CTA of variant 11 (0
+ * picks its default, which at finalize counts the injection terms;
+ * FDTD_ERR_INVALID_ARG when a CTA cannot hold them); the other variants ignore it.
+ * Autotuning an engine that runs 11 picks its tile. */
 int fdtd_engine_set_launch(fdtd_engine* h, int variant, int tile_rows, int chunk_planes);
 int fdtd_engine_get_launch(fdtd_engine* h, int* variant, int* tile_rows, int* chunk_planes);
 /* Where the Debye / Drude / Lorentz poles advance: on (1, the default) in a

@@ -242,8 +242,8 @@ def test_spectra_equal_the_scaled_accumulators(bloch):
 
 
 def test_released_memory_goes_back_to_the_device():
-    """A closed solver's arrays stay in the pool (a second one of the same scene takes
-    them from there) until they are given back."""
+    """A closed solver's arrays stay with torch's allocator (a second one of the same
+    scene takes them from there) until they are given back."""
     import torch
 
     wm = load_package()
@@ -253,7 +253,7 @@ def test_released_memory_goes_back_to_the_device():
     for _ in range(2):
         solver = wm.solver.B200FDTD(cs).init_field()
         solver.step_range(0, 2)
-        assert float(solver.field("Ez").abs().max()) == 0.0  # pooled memory starts at zero too
+        assert float(solver.field("Ez").abs().max()) == 0.0  # reused memory starts at zero too
         solver.set_field("Ez", torch.ones(wm.scene.component_shape("Ez", cs.nodes), device="cuda"))
         solver.close()
     wm.solver.release_memory()

@@ -1103,6 +1103,9 @@ int term_planes(const fdtd_engine* h, int planes) {
 //   ends last: 0.6 us a term and plane (24 dipoles over the same cells of 257^3: 426 us
 //   at 29 planes, 180 at 6; 8 of them: 211 and 144).  One or two cost less than
 //   shorter chunks do (193^3, one: 63.5 us at 13 planes, 65.5 at 10).
+// Rows of 389 to 512 nodes, which with CPML leave a CTA three to five rows beside the
+// one that it recomputes: 257 x 257 x 501, 12 cells, 508 us (warp kernel 718); 161 x 161
+// x 512, 10 cells, 230 (315).
 void default_quad(fdtd_engine* h, int ty, int cx) {
   const int Q = h->P / 4;
   double best = 1e300;
