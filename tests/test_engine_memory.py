@@ -165,7 +165,7 @@ def test_an_allocator_that_fails_is_an_error_and_leaves_nothing_behind():
         del held[memory]
 
     desc = wm._lib.FdtdGridDesc()
-    desc.nx = desc.ny = desc.nz = 17
+    desc.nx = desc.ny = desc.nz = 33
     desc.dt = 4e-17
     handle = ctypes.c_void_p()
     rc = lib.fdtd_engine_create_with(ctypes.byref(desc), None, alloc, release, None, ctypes.byref(handle))
