@@ -25,6 +25,7 @@
 #ifndef FDTD_B200_H
 #define FDTD_B200_H
 
+#include <stddef.h>
 #include <stdint.h>
 
 #ifdef __cplusplus
